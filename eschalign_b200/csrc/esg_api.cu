@@ -54,10 +54,43 @@ esg_status cuda_fail(cudaError_t e, const char* what) {
 constexpr uint32_t kMaxRefLen = 32768;
 // device memory k3's column buffers may take (per scorer and arm)
 constexpr size_t kColbufBudget = (size_t)1 << 30;
+// Dynamic shared memory of a k2 CTA at most: three CTAs' worth of an SM, the
+// 28- and 32-row kernels' occupancy by registers.  A larger panel is read
+// through L2, which costs less than a CTA.
+constexpr size_t kK2SmemLimit = 74 * 1024;
 constexpr int kPad = 5;     // selector / table index of a padding column or row
 constexpr int kWild = 4;
 
 inline uint32_t code_of(uint8_t c) { return c > 4 ? 4u : c; }
+
+// k2's shapes: tiles of 8-, 16-, 28- and 32-row stripes, and one long query in
+// passes of 32 32-row stripes.  A batch's tasks lie in the order long, 32,
+// 28, 16, 8.
+enum K2Shape { kLongQuery = 0, kRows32, kRows28, kRows16, kRows8, kShapes };
+constexpr uint32_t kStripeRows[kShapes] = {32, 32, 28, 16, 8};
+
+// The shape of a query of n rows past the split: the one with the least
+// work.  A stripe carries per-column work of about 3.7 rows (the column's
+// selector and record, the top input), so a row costs 1.112 on 16-row and
+// 1.045 on 28-row stripes against 1 on 32-row ones (C2 local, 150 000 reads
+// all on one shape, less their padding: 118.9, 111.7, 106.9 ms); a shorter
+// stripe wins where it pads enough less: n = 110 takes 112 rows of 28
+// against 128.  The shapes together: 115.8 ms against 121.2 (32 rows alone)
+// and 126.9 (16 alone).  From 225 rows on the padding is under 6 % and one
+// shape's tiles pack better than two's (50-1000 nt reads against 3000
+// references: 208 ms against 217 with 28-row stripes at every length).
+K2Shape shape_of(uint32_t n) {
+  if (n > 32u * 32u) return kLongQuery;
+  if (n > 28u * 8u) return kRows32;
+  return (n + 27) / 28 * 28 * 1045 < (n + 31) / 32 * 32 * 1000 ? kRows28 : kRows32;
+}
+
+// Panel chunks per tile at most, unless esg_scorer_set_chunking says less.
+constexpr uint32_t kMaxChunks = 1024;
+
+// A batch's device counters: [1] re-score requests, [2] error bits, [6..7]
+// k3's 64-bit unit counter, one task counter per k2 shape in the others.
+constexpr uint32_t kCounters = 9;
 
 // Pinned host memory, reused across batches of one scorer.
 struct PinnedPool {
@@ -111,7 +144,6 @@ struct esg_scorer {
   uint32_t n_refs = 0;
   uint32_t max_ref_len = 0;
   uint64_t panel_bases = 0;
-  bool panel_w = false;
   bool batched_ok = false;
   // k2 panel
   uint32_t n_pairs = 0;
@@ -121,32 +153,35 @@ struct esg_scorer {
   void* d_blob = nullptr;
   std::vector<uint64_t> pair_cols;  // prefix sums of the pairs' column counts
   uint32_t tab_a[6]{}, tab_b[6]{};
+  uint32_t tabh_a[6]{}, tabh_b[6]{};  // kLanesHalf: s + half_off per byte
+  bool half_ok = false;               // local, and the scheme fits those tables
+  int half_off = 0;
   int sat = 0;
   size_t k2_smem = 0;
   uint2* d_lbuf = nullptr;   // long queries: one column buffer per k2 warp
   uint32_t lbuf_cols = 0;
-  const void* k2_t16 = nullptr;   // tiles of 16-row stripes
-  const void* k2_t32 = nullptr;   // tiles of 32-row stripes
-  const void* k2_long = nullptr;  // one long query, 32-row stripes, in passes
-  int blocks_t16 = 0, blocks_t32 = 0, blocks_long = 0;
-  // semi-global: the same three with every cell's maximum checked against
-  // the int16 lanes' upper limit, for batches holding queries past the
-  // static bound (k2_checks)
-  const void* k2c_t16 = nullptr;
-  const void* k2c_t32 = nullptr;
-  const void* k2c_long = nullptr;
-  int blocksc_t16 = 0, blocksc_t32 = 0, blocksc_long = 0;
-  // queries up to split_len bases take 16-row stripes, longer ones 32-row
-  // stripes (esg_scorer_autotune measures where 32 rows start to win)
-  uint32_t split_len = 256;
+  // The kernels of each shape: [0], and a second one.  Semi-global: every
+  // cell's maximum checked against the int16 lanes' upper limit, for batches
+  // holding queries past the static bound (k2_checks).  Local: f16 lanes, for
+  // task groups whose queries stay inside them (k2_half).
+  struct K2Kernel {
+    const void* fn = nullptr;
+    int blocks = 0;      // CTAs launched at most
+    int occupancy = 0;   // the same, all that fit (the autotuner may lower blocks)
+  };
+  K2Kernel k2[kShapes][2];
+  // queries up to split_len bases take 16-row stripes, longer ones what
+  // shape_of gives (esg_scorer_autotune measures where that starts to win)
+  uint32_t split_len = 16;
   bool tuned = false;
+  bool split_set = false;   // by esg_scorer_set_split, or the autotuner at work
   // queries of this length and longer go to the int32 lanes instead of the
   // batched kernel (0: none; set by the autotuner where the batched kernel
   // would flag most of them)
   uint32_t int32_from = 0;
   // panel chunking aims for this many tasks per resident warp
   uint32_t chunk_target = 8;
-  uint32_t max_chunks = 64;  // panel chunks per tile at most (1: never chunk)
+  uint32_t max_chunks = kMaxChunks;  // panel chunks per tile at most (1: never chunk)
   cudaStream_t aux = nullptr;          // second stream: the long-query kernel
   // batches' device memory: a pool of this scorer's own that keeps what
   // finished batches return, so the next batch maps no new memory
@@ -192,14 +227,12 @@ struct esg_batch {
   std::vector<uint64_t> exceptions;
   // host plan
   uint32_t n_tasks = 0;
-  uint32_t n_long = 0;   // tasks are [n_long long | n_t32 tiles | n_t16 tiles]
-  uint32_t n_t32 = 0;
-  uint32_t n_t16 = 0;
+  uint32_t n_tiles[kShapes] = {};      // tasks of each shape, in that order
+  bool second[kShapes] = {};           // the shape's second kernel runs them
   uint32_t n_order = 0;
   uint32_t host_list = 0;
   uint32_t redo_cap = 0;
   uint32_t n_chunks = 1;  // panel chunks per tile (k2 tasks = tiles x chunks)
-  bool sg_check = false;  // semi-global: run the checked k2 variants
   // paired batches (esg_prepare_pairs): reads 2p, 2p + 1 are pair p's mates
   bool paired = false;
   bool pair_both = false;   // rank both template strands
@@ -288,6 +321,14 @@ bool k2_checks(const esg_scorer* sc, uint64_t n) {
   return value_bound(n, sc->max_ref_len, sc->scoring) + mm >= 12000;
 }
 
+// Local queries whose every score fits the f16 lanes' whole numbers.  With
+// the common schemes (match 1 or 2) that is every read up to 1023 bases, and
+// longer ones against a panel of shorter references.
+bool k2_half(const esg_scorer* sc, uint64_t n) {
+  return sc->half_ok && (int64_t)std::min<uint64_t>(n, sc->max_ref_len) *
+                                sc->scoring.match_score <= kHalfMax;
+}
+
 bool k2_takes(const esg_scorer* sc, uint64_t n) {
   if (!sc->batched_ok || n == 0) return false;
   // queries over 32 stripes of 32 rows run in passes chained through the
@@ -314,30 +355,34 @@ T* carve(char*& at, size_t count) {
 
 size_t carve_size(size_t count, size_t elem) { return (count * elem + 255) / 256 * 256; }
 
-template <int R, bool kLong, bool kLocal, bool kCheck>
-const void* pick_k2_ws(bool w, bool smem) {
-  if (w)
-    return smem ? (const void*)k2_batched<R, kLocal, true, true, kLong, kCheck>
-                : (const void*)k2_batched<R, kLocal, true, false, kLong, kCheck>;
-  return smem ? (const void*)k2_batched<R, kLocal, false, true, kLong, kCheck>
-              : (const void*)k2_batched<R, kLocal, false, false, kLong, kCheck>;
-}
-
 template <int R, bool kLong>
-const void* pick_k2(bool local, bool check, bool w, bool smem) {
-  if (local) return pick_k2_ws<R, kLong, true, false>(w, smem);
-  return check ? pick_k2_ws<R, kLong, false, true>(w, smem)
-               : pick_k2_ws<R, kLong, false, false>(w, smem);
+const void* pick_k2(bool local, int lanes, bool smem) {
+  if (lanes == kLanesHalf)
+    return smem ? (const void*)k2_batched<R, true, true, kLong, kLanesHalf>
+                : (const void*)k2_batched<R, true, false, kLong, kLanesHalf>;
+  if (local)
+    return smem ? (const void*)k2_batched<R, true, true, kLong, kLanesInt>
+                : (const void*)k2_batched<R, true, false, kLong, kLanesInt>;
+  if (lanes == kLanesChecked)
+    return smem ? (const void*)k2_batched<R, false, true, kLong, kLanesChecked>
+                : (const void*)k2_batched<R, false, false, kLong, kLanesChecked>;
+  return smem ? (const void*)k2_batched<R, false, true, kLong, kLanesInt>
+              : (const void*)k2_batched<R, false, false, kLong, kLanesInt>;
 }
 
 void set_k2_fn(esg_scorer* sc) {
-  const bool local = sc->mode == ESG_MODE_LOCAL;
-  sc->k2_t16 = pick_k2<16, false>(local, false, sc->panel_w, sc->smem_panel);
-  sc->k2_t32 = pick_k2<32, false>(local, false, sc->panel_w, sc->smem_panel);
-  sc->k2_long = pick_k2<32, true>(local, false, sc->panel_w, sc->smem_panel);
-  sc->k2c_t16 = pick_k2<16, false>(local, !local, sc->panel_w, sc->smem_panel);
-  sc->k2c_t32 = pick_k2<32, false>(local, !local, sc->panel_w, sc->smem_panel);
-  sc->k2c_long = pick_k2<32, true>(local, !local, sc->panel_w, sc->smem_panel);
+  const bool local = sc->mode == ESG_MODE_LOCAL, smem = sc->smem_panel;
+  // the second kernel of a mode (k2_second): local, f16 lanes where the
+  // scheme fits them; semi-global, the checked lanes
+  const int second = !local ? kLanesChecked : sc->half_ok ? kLanesHalf : kLanesInt;
+  for (int w = 0; w < 2; ++w) {
+    const int lanes = w ? second : kLanesInt;
+    sc->k2[kLongQuery][w].fn = pick_k2<32, true>(local, lanes, smem);
+    sc->k2[kRows32][w].fn = pick_k2<32, false>(local, lanes, smem);
+    sc->k2[kRows28][w].fn = pick_k2<28, false>(local, lanes, smem);
+    sc->k2[kRows16][w].fn = pick_k2<16, false>(local, lanes, smem);
+    sc->k2[kRows8][w].fn = pick_k2<8, false>(local, lanes, smem);
+  }
   sc->k3_fn = local ? (const void*)k3_lanes<true> : (const void*)k3_lanes<false>;
 }
 
@@ -568,9 +613,6 @@ esg_status esg_scorer_new(int32_t device, const uint8_t* ref_codes, const uint64
   for (uint32_t r = 0; r < n_refs; ++r) order[r] = r;
   std::stable_sort(order.begin(), order.end(),
                    [&](uint32_t a, uint32_t b) { return ref_len[a] > ref_len[b]; });
-  for (uint32_t r = 0; r < n_refs; ++r)
-    for (uint32_t j = 0; j < ref_len[r]; ++j)
-      if (code_of(ref_codes[ref_off[r] + j]) == kWild) sc->panel_w = true;
 
   // --- scoring tables of the batched kernel: s - o as int8 per byte
   const int ma = s.match_score, mi = s.mismatch, o = s.gap_open;
@@ -594,6 +636,20 @@ esg_status esg_scorer_new(int32_t device, const uint8_t* ref_codes, const uint64
     // local: a best H at or above this may have left the int16 lanes (the
     // diagonal term reaches H + ma + bias); such queries are re-scored in int32
     sc->sat = 32767 - ma - kBiasLocal;
+    // f16 lanes: bytes s + half_off in 0..127 (the selectors' sign fill is
+    // then 0), half_off taken off again per record; a padding column's byte
+    // is 0, the worst score, at most 0
+    sc->half_off = std::max(0, -mi);
+    sc->half_ok = mode == ESG_MODE_LOCAL && ma + sc->half_off <= 127;
+    if (sc->half_ok) {
+      for (int c = 0; c < 6; ++c) {
+        uint32_t a = 0;
+        for (int x = 0; x < 4; ++x)
+          a |= (uint32_t)((c == kWild || c == x ? ma : mi) + sc->half_off) << (8 * x);
+        sc->tabh_a[c] = a;
+        sc->tabh_b[c] = (uint32_t)(ma + sc->half_off);
+      }
+    }
   }
 
   // --- reference pairs and their selectors
@@ -619,8 +675,8 @@ esg_status esg_scorer_new(int32_t device, const uint8_t* ref_codes, const uint64
     sc->pair_cols[p + 1] = sc->pair_cols[p] + (pairs[p].y & 0xffffu);
   sc->sel_base = sc->n_pairs * 8;  // uint16 units after the pair table
   const size_t raw = (size_t)sc->n_pairs * 16 + sels.size() * 2;
-  // one spare selector past the last pair: a lane may load column m
-  sc->blob_bytes = (uint32_t)((raw + 2 + 15) / 16 * 16);
+  // two spare selectors past the last pair: a lane may load columns m, m + 1
+  sc->blob_bytes = (uint32_t)((raw + 4 + 15) / 16 * 16);
   std::vector<unsigned char> blob(sc->blob_bytes, 0);
   memcpy(blob.data(), pairs.data(), pairs.size() * 16);
   memcpy(blob.data() + (size_t)sc->n_pairs * 16, sels.data(), sels.size() * 2);
@@ -669,14 +725,16 @@ esg_status esg_scorer_new(int32_t device, const uint8_t* ref_codes, const uint64
 
   // --- launch geometry
   const size_t slots = (size_t)kK2Threads * (4 + cap + kScrWords) * 4;
-  sc->smem_panel = (size_t)sc->blob_bytes + slots <= 100 * 1024;
+  sc->smem_panel = (size_t)sc->blob_bytes + slots <= kK2SmemLimit;
   set_k2_fn(sc);
   sc->k2_smem = (sc->smem_panel ? sc->blob_bytes : 0) + slots;
-  for (const void* fn : {sc->k2_t16, sc->k2_t32, sc->k2_long, sc->k2c_t16, sc->k2c_t32,
-                         sc->k2c_long})
-    if ((e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)sc->k2_smem)) != cudaSuccess)
-      return cleanup(cuda_fail(e, "cudaFuncSetAttribute(k2)"));
+  // (the attribute is the process's: every scorer sets the same limit, or
+  // one over a smaller panel would take it from the others)
+  for (auto& shape : sc->k2)
+    for (auto& k : shape)
+      if ((e = cudaFuncSetAttribute(k.fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    (int)kK2SmemLimit)) != cudaSuccess)
+        return cleanup(cuda_fail(e, "cudaFuncSetAttribute(k2)"));
   if ((e = cudaStreamCreateWithFlags(&sc->aux, cudaStreamNonBlocking)) != cudaSuccess ||
       (e = cudaEventCreateWithFlags(&sc->fork, cudaEventDisableTiming)) != cudaSuccess ||
       (e = cudaEventCreateWithFlags(&sc->join, cudaEventDisableTiming)) != cudaSuccess)
@@ -693,36 +751,24 @@ esg_status esg_scorer_new(int32_t device, const uint8_t* ref_codes, const uint64
         cudaSuccess)
       return cleanup(cuda_fail(e, "cudaMemPoolSetAttribute"));
   }
-  int occ16 = 0, occ32 = 0, occl = 0, occ3 = 0;
-  if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ16, sc->k2_t16, kK2Threads,
-                                                         sc->k2_smem)) != cudaSuccess ||
-      (e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ32, sc->k2_t32, kK2Threads,
-                                                         sc->k2_smem)) != cudaSuccess ||
-      (e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occl, sc->k2_long, kK2Threads,
-                                                         sc->k2_smem)) != cudaSuccess ||
-      (e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ3, sc->k3_fn, kK3Threads, 0)) !=
-          cudaSuccess)
+  int occ3 = 0;
+  if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ3, sc->k3_fn, kK3Threads, 0)) !=
+      cudaSuccess)
     return cleanup(cuda_fail(e, "cudaOccupancy"));
-  sc->blocks_t16 = std::max(1, occ16) * sc->sm_count;
-  sc->blocks_t32 = std::max(1, occ32) * sc->sm_count;
-  sc->blocks_long = std::max(1, occl) * sc->sm_count;
-  {
-    int c16 = 0, c32 = 0, cl = 0;
-    if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&c16, sc->k2c_t16, kK2Threads,
-                                                           sc->k2_smem)) != cudaSuccess ||
-        (e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&c32, sc->k2c_t32, kK2Threads,
-                                                           sc->k2_smem)) != cudaSuccess ||
-        (e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&cl, sc->k2c_long, kK2Threads,
-                                                           sc->k2_smem)) != cudaSuccess)
-      return cleanup(cuda_fail(e, "cudaOccupancy"));
-    sc->blocksc_t16 = std::max(1, c16) * sc->sm_count;
-    sc->blocksc_t32 = std::max(1, c32) * sc->sm_count;
-    // the long-query column buffer below is sized for blocks_long CTAs
-    sc->blocksc_long = std::min(std::max(1, cl) * sc->sm_count, sc->blocks_long);
-  }
+  for (auto& shape : sc->k2)
+    for (auto& k : shape) {
+      int occ = 0;
+      if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k.fn, kK2Threads,
+                                                             sc->k2_smem)) != cudaSuccess)
+        return cleanup(cuda_fail(e, "cudaOccupancy"));
+      k.blocks = k.occupancy = std::max(1, occ) * sc->sm_count;
+    }
+  // the long-query column buffer below is sized for the first kernel's CTAs
+  sc->k2[kLongQuery][1].blocks =
+      std::min(sc->k2[kLongQuery][1].blocks, sc->k2[kLongQuery][0].blocks);
   if (sc->batched_ok && max_len <= 8192) {
     sc->lbuf_cols = max_len;
-    const size_t lb = (size_t)sc->blocks_long * kK2Warps * max_len * sizeof(uint2);
+    const size_t lb = (size_t)sc->k2[kLongQuery][0].blocks * kK2Warps * max_len * sizeof(uint2);
     if ((e = cudaMalloc(&sc->d_lbuf, lb)) != cudaSuccess)
       return cleanup(cuda_fail(e, "cudaMalloc(long-query buffer)"));
   }
@@ -755,7 +801,7 @@ esg_status esg_scorer_new(int32_t device, const uint8_t* ref_codes, const uint64
   inf.panel_bytes = sc->smem_panel ? sc->blob_bytes : 0;
   inf.batched_ok = sc->batched_ok;
   cudaFuncAttributes fa{};
-  if (cudaFuncGetAttributes(&fa, sc->k2_t16) == cudaSuccess) {
+  if (cudaFuncGetAttributes(&fa, sc->k2[kRows16][0].fn) == cudaSuccess) {
     inf.regs_batched = fa.numRegs;
     inf.local_bytes_batched = (int)fa.localSizeBytes;
   }
@@ -763,7 +809,7 @@ esg_status esg_scorer_new(int32_t device, const uint8_t* ref_codes, const uint64
     inf.regs_plain = fa.numRegs;
     inf.local_bytes_plain = (int)fa.localSizeBytes;
   }
-  inf.batched_blocks = sc->blocks_t16;
+  inf.batched_blocks = sc->k2[kRows16][0].blocks;
   inf.batched_threads = kK2Threads;
   inf.plain_blocks = sc->k3_blocks;
   inf.plain_threads = kK3Threads;
@@ -836,6 +882,7 @@ esg_status esg_scorer_set_chunking(esg_scorer* sc, uint32_t max_chunks) {
 esg_status esg_scorer_set_split(esg_scorer* sc, uint32_t split_len) {
   if (!sc) return fail(ESG_ERR_BAD_ARGUMENT, "NULL scorer");
   sc->split_len = split_len;
+  sc->split_set = true;
   sc->info.split_len = split_len;
   return ESG_OK;
 }
@@ -914,8 +961,8 @@ static esg_status autotune_impl(esg_scorer* sc, const std::vector<uint32_t>& his
   if (!sc) return fail(ESG_ERR_BAD_ARGUMENT, "NULL scorer");
   esg_tune_report rep{};
   rep.chunk_target = sc->chunk_target;
-  rep.ctas16 = sc->blocks_t16 / std::max(1, sc->sm_count);
-  rep.ctas32 = sc->blocks_t32 / std::max(1, sc->sm_count);
+  rep.ctas16 = sc->k2[kRows16][0].blocks / std::max(1, sc->sm_count);
+  rep.ctas32 = sc->k2[kRows32][0].blocks / std::max(1, sc->sm_count);
   if (!sc->batched_ok || sc->kernel != ESG_KERNEL_AUTO) {
     rep.split_len = sc->split_len;
     rep.int32_from = sc->int32_from;
@@ -926,14 +973,17 @@ static esg_status autotune_impl(esg_scorer* sc, const std::vector<uint32_t>& his
   static const uint32_t kLens[] = {48, 80, 112, 160, 224, 320, 448};
   const uint32_t n_lens = sizeof(kLens) / sizeof(kLens[0]);
   const uint32_t keep_split = sc->split_len, keep_from = sc->int32_from;
-  const int keep16 = sc->blocks_t16, keep32 = sc->blocks_t32;
+  esg_scorer::K2Kernel keep_k2[kShapes][2];
+  std::copy(&sc->k2[0][0], &sc->k2[0][0] + kShapes * 2, &keep_k2[0][0]);
   const uint32_t keep_target = sc->chunk_target;
+  const bool keep_set = sc->split_set;
+  sc->split_set = true;
   auto restore = [&]() {
+    sc->split_set = keep_set;
     sc->split_len = keep_split;
     sc->int32_from = keep_from;
     sc->kernel = ESG_KERNEL_AUTO;
-    sc->blocks_t16 = keep16;
-    sc->blocks_t32 = keep32;
+    std::copy(&keep_k2[0][0], &keep_k2[0][0] + kShapes * 2, &sc->k2[0][0]);
     sc->chunk_target = keep_target;
   };
   uint64_t x = 0x9e3779b97f4a7c15ull;
@@ -1029,15 +1079,21 @@ static esg_status autotune_impl(esg_scorer* sc, const std::vector<uint32_t>& his
     const uint32_t L = which == 0 ? 112u : 448u;
     calib_reads(sc, L, reads_for(L), x, c);
     sc->split_len = which == 0 ? 512u : 0u;
-    int& blocks = which == 0 ? sc->blocks_t16 : sc->blocks_t32;
-    const int occ = (which == 0 ? keep16 : keep32) / std::max(1, sc->sm_count);
+    // (each kernel up to its own occupancy; the 28-row ones with the 32-row)
+    int occ = 1;
+    for (const auto& k : sc->k2[which == 0 ? kRows16 : kRows32])
+      occ = std::max(occ, k.occupancy / std::max(1, sc->sm_count));
+    auto set_blocks = [&](int n) {
+      for (int shape : {which == 0 ? kRows16 : kRows32, which == 0 ? kRows16 : kRows28})
+        for (auto& k : sc->k2[shape]) k.blocks = std::min(n * sc->sm_count, k.occupancy);
+    };
     uint32_t* cand = which == 0 ? rep.cand_ctas16 : rep.cand_ctas32;
     float* tms = which == 0 ? rep.ms_ctas16 : rep.ms_ctas32;
     uint32_t& n_c = which == 0 ? rep.n_ctas16 : rep.n_ctas32;
     float best = 0;
     int pick = occ;
     for (int k = occ; k >= std::max(1, occ - 2) && st == ESG_OK; --k) {
-      blocks = k * sc->sm_count;
+      set_blocks(k);
       float ms = 0;
       st = time_calib(sc, c, e0, e1, &ms);
       cand[n_c] = (uint32_t)k;
@@ -1048,14 +1104,14 @@ static esg_status autotune_impl(esg_scorer* sc, const std::vector<uint32_t>& his
         pick = k;
       }
     }
-    blocks = pick * sc->sm_count;
+    set_blocks(pick);
     (which == 0 ? rep.ctas16 : rep.ctas32) = (uint32_t)pick;
   }
   sc->split_len = split;
   // 3. panel chunking: a batch of about one read per resident warp (too few
   //    tiles to fill the GPU), chunked to aim for 1-16 tasks per resident warp
   if (st == ESG_OK) {
-    calib_reads(sc, 112, (uint32_t)std::max(64, sc->blocks_t16 * kK2Warps), x, c);
+    calib_reads(sc, 112, (uint32_t)std::max(64, sc->k2[kRows16][0].blocks * kK2Warps), x, c);
     static const uint32_t kTargets[] = {1, 2, 4, 8, 16};
     float best = 0;
     uint32_t pick = keep_target;
@@ -1082,11 +1138,12 @@ static esg_status autotune_impl(esg_scorer* sc, const std::vector<uint32_t>& his
     return st;
   }
   sc->split_len = split;
+  sc->split_set = false;
   sc->int32_from = from;
   sc->tuned = true;
   sc->info.split_len = split;
   sc->info.tuned = 1;
-  sc->info.batched_blocks = sc->blocks_t16;
+  sc->info.batched_blocks = sc->k2[kRows16][0].blocks;
   rep.split_len = split;
   rep.int32_from = from;
   if (out) *out = rep;
@@ -1198,11 +1255,35 @@ static esg_status prepare_impl(esg_scorer* sc, const uint8_t* const* ptrs, const
   // longer ones 32-row stripes (from sc->split_len, set by the autotuner),
   // queries over 32 stripes of 32 rows run alone in passes; what the
   // batched kernel cannot take goes to the int32 kernel.
-  std::vector<std::pair<uint32_t, uint32_t>> q16, q32, qlong;  // (stripes, query)
+  std::vector<std::pair<uint32_t, uint32_t>> qs[kShapes];  // (stripes, query)
   std::vector<uint8_t> route(b->n_q, 0);  // 0 empty or k2, 2 k3
+  bool sg_check = false, half[kShapes] = {true, true, true, true, true};
   uint32_t n_k3 = 0, n_empty = 0, redo_cap = 0;
   uint64_t cells = 0;
   const uint32_t split = std::min<uint32_t>(sc->split_len, 16 * kMaxStripes);
+  // Batches too small to fill the GPU: what counts is the time of one column,
+  // about 13 cycles a row (the F chain) and 45 more, not the lanes it fills.
+  // Short stripes then win as long as their (tile, reference pair) tasks fit
+  // the SMs' schedulers side by side: 8 rows up to two a scheduler, 16 rows
+  // up to six.  Device time against 164 references, reads of ~110 nt on 28 /
+  // 32, 16 and 8 rows: 1 read 68, 44, 32 us; 16 reads 73, 57, 82 us (8 rows:
+  // 2.8 a scheduler); 61 reads 107, 100 us (16 rows: 4.7).
+  int short_shape = kRows16;
+  uint32_t short_cap = 0;
+  if (!sc->split_set) {
+    uint64_t s8 = 0, s16 = 0;
+    for (uint32_t k = 0; k < n_reads; ++k) {
+      s8 += std::min<uint32_t>((len[k] + 7) / 8, kMaxStripes);
+      s16 += std::min<uint32_t>((len[k] + 15) / 16, kMaxStripes);
+    }
+    const uint64_t tasks = (uint64_t)sc->n_pairs * (both ? 2 : 1), scheds = 4ull * sc->sm_count;
+    if ((s8 * tasks + 31) / 32 <= 2 * scheds) {
+      short_shape = kRows8;
+      short_cap = 8 * kMaxStripes;
+    } else if ((s16 * tasks + 31) / 32 <= 6 * scheds) {
+      short_cap = 16 * kMaxStripes;
+    }
+  }
   for (uint32_t q = 0; q < b->n_q; ++q) {
     const uint32_t n = len[q < n_reads ? q : q - n_reads];
     if (n == 0) {
@@ -1212,14 +1293,12 @@ static esg_status prepare_impl(esg_scorer* sc, const uint8_t* const* ptrs, const
     cells += (uint64_t)n * sc->panel_bases;
     const bool lanes32 = sc->int32_from && n >= sc->int32_from;
     if (b->kernel == ESG_KERNEL_AUTO && !lanes32 && k2_takes(sc, n)) {
-      if (n <= split)
-        q16.push_back({(n + 15) / 16, q});
-      else if (n <= 32 * kMaxStripes)
-        q32.push_back({(n + 31) / 32, q});
-      else
-        qlong.push_back({(n + 31) / 32, q});
+      const int shape = n <= short_cap ? short_shape : n <= split ? kRows16 : shape_of(n);
+      const uint32_t R = kStripeRows[shape];
+      qs[shape].push_back({(n + R - 1) / R, q});
       if (k2_may_flag(sc, n)) ++redo_cap;
-      if (k2_checks(sc, n)) b->sg_check = true;
+      if (k2_checks(sc, n)) sg_check = true;
+      if (!k2_half(sc, n)) half[shape] = false;
     } else {
       route[q] = 2;
       ++n_k3;
@@ -1227,29 +1306,35 @@ static esg_status prepare_impl(esg_scorer* sc, const uint8_t* const* ptrs, const
   }
   b->host_list = n_k3;
   b->redo_cap = redo_cap;
+  const bool local = sc->mode == ESG_MODE_LOCAL;
+  for (int k = 0; k < kShapes; ++k) b->second[k] = local ? half[k] : sg_check;
+  auto& qlong = qs[kLongQuery];
   std::stable_sort(qlong.begin(), qlong.end(),
                    [](const std::pair<uint32_t, uint32_t>& a,
                       const std::pair<uint32_t, uint32_t>& c) { return a.first > c.first; });
-  TilePlan p32, p16;
-  pack_tiles(q32, p32);
-  pack_tiles(q16, p16);
-  const uint32_t n_long = (uint32_t)qlong.size();
-  b->n_long = n_long;
-  b->n_t32 = (uint32_t)p32.tasks.size();
-  b->n_t16 = (uint32_t)p16.tasks.size();
-  b->n_tasks = b->n_long + b->n_t32 + b->n_t16;
-  b->n_order = n_long + (uint32_t)(q32.size() + q16.size());
+  TilePlan plans[kShapes];
+  b->n_tiles[kLongQuery] = (uint32_t)qlong.size();
+  for (int k = kRows32; k < kShapes; ++k) {
+    pack_tiles(qs[k], plans[k]);
+    b->n_tiles[k] = (uint32_t)plans[k].tasks.size();
+  }
+  for (int k = 0; k < kShapes; ++k) {
+    b->n_tasks += b->n_tiles[k];
+    b->n_order += (uint32_t)qs[k].size();
+  }
   // --- panel chunks: when the tiles are too few to keep every resident warp
   // busy to the end (few reads, or a large panel), each tile's reference
-  // pairs are cut into chunks of about equal columns, one task each, and
-  // the per-chunk query states are merged afterwards
+  // pairs are cut into chunks of about equal columns, one task each, down to
+  // one pair, and the per-chunk query states are merged afterwards (one read
+  // against 164 references: 123 us in chunks of four pairs or more, 68 in
+  // chunks of one; 500 reads 598 -> 471)
   {
     const uint64_t tiles = b->n_tasks;
     const uint64_t target =
-        (uint64_t)sc->chunk_target * (uint64_t)std::max(sc->blocks_t16, 1) * kK2Warps;
+        (uint64_t)sc->chunk_target * (uint64_t)std::max(sc->k2[kRows16][0].blocks, 1) * kK2Warps;
     uint32_t nc = 1;
     if (tiles && tiles < target) nc = (uint32_t)((target + tiles - 1) / tiles);
-    nc = std::min<uint32_t>(nc, std::max<uint32_t>(1, sc->n_pairs / 4));
+    nc = std::min<uint32_t>(nc, sc->n_pairs);
     nc = std::min<uint32_t>(nc, sc->max_chunks);
     b->n_chunks = std::max<uint32_t>(nc, 1);
   }
@@ -1316,7 +1401,8 @@ static esg_status prepare_impl(esg_scorer* sc, const uint8_t* const* ptrs, const
       b->h_tasks[t++] = make_uint2(o++, 1u | (lq.first << 16));
       lanes += lq.first;
     }
-    for (const TilePlan* tp : {&p32, &p16}) {
+    for (int k = kRows32; k < kShapes; ++k) {
+      const TilePlan* tp = &plans[k];
       const uint32_t base = o;
       for (uint32_t q : tp->order) b->h_order[o++] = q;
       for (const uint2& tk : tp->tasks) b->h_tasks[t++] = make_uint2(base + tk.x, tk.y);
@@ -1332,7 +1418,7 @@ static esg_status prepare_impl(esg_scorer* sc, const uint8_t* const* ptrs, const
   b->stats.n_reads = n_reads;
   b->stats.n_queries = b->n_q;
   b->stats.n_empty = n_empty;
-  b->stats.queries_batched = n_long + (uint32_t)(q32.size() + q16.size());
+  b->stats.queries_batched = b->n_order;
   b->stats.queries_plain = n_k3;
   b->stats.tasks = b->n_tasks;
   b->stats.panel_chunks = b->n_chunks;
@@ -1415,12 +1501,12 @@ static size_t batch_device_bytes(const esg_scorer* sc, const esg_batch* b) {
       carve_size(b->n_tasks ? b->n_tasks : 1, 8),
       carve_size(nlist ? nlist : 1, 4),
       carve_size(b->n_chunks + 1, 4),
-      carve_size(8, 4),
       carve_size(nq, 16),
       carve_size(nq * sc->cap, 4),
       carve_size(nlist ? (size_t)nlist * sc->n_refs : 1, 4),
       carve_size(nr, 16),
       carve_size(nr * sc->cap, 4),
+      carve_size(kCounters, 4),
       dev_rows ? carve_size(nq * sc->n_refs, 4) : 0,
       carve_size(2 * np, 16),
       carve_size(np * sc->cap, 4),
@@ -1433,11 +1519,17 @@ static size_t batch_device_bytes(const esg_scorer* sc, const esg_batch* b) {
 }
 
 // ---------------------------------------------------------------- device work
+static bool fused_merge(const esg_batch* b) {
+  return b->n_chunks > 1 && b->n_tasks && b->host_list + b->redo_cap == 0;
+}
+
 static esg_status launch_device_work(esg_scorer* sc, esg_batch* b, cudaStream_t st) {
   const bool both = b->flags & ESG_BOTH_STRANDS;
   uint32_t kernels = 0;
   const bool rows = b->d_rows != nullptr;
-  ESG_CUDA(cudaMemsetAsync(b->d_counters, 0, 8 * sizeof(uint32_t), st));
+  // chunked, and nothing for k3: the chunks' states go straight to the results
+  const bool fused = fused_merge(b);
+  ESG_CUDA(cudaMemsetAsync(b->d_counters, 0, kCounters * sizeof(uint32_t), st));
   if (b->n_tasks) {
     K2Params P{};
     P.blob = (const uint4*)sc->d_blob;
@@ -1465,6 +1557,7 @@ static esg_status launch_device_work(esg_scorer* sc, esg_batch* b, cudaStream_t 
     P.part_ties = b->d_part_ties;
     memcpy(P.tab_a, sc->tab_a, sizeof P.tab_a);
     memcpy(P.tab_b, sc->tab_b, sizeof P.tab_b);
+    P.borrow = sc->scoring.mismatch < sc->scoring.gap_open;
     P.e2 = pack16x2(sc->scoring.gap_extend, sc->scoring.gap_extend);
     P.o = sc->scoring.gap_open;
     P.e = sc->scoring.gap_extend;
@@ -1474,62 +1567,48 @@ static esg_status launch_device_work(esg_scorer* sc, esg_batch* b, cudaStream_t 
     P.lbuf_cols = sc->lbuf_cols;
     P.sat = sc->sat;
     P.cap = sc->cap;
-    // The three task groups: long queries, then 32-row tiles, on the aux
-    // stream; 16-row tiles on the batch's stream.  Launched first, the aux
-    // kernels' CTAs share the SMs with the persistent 16-row kernel and
-    // fill its tail, instead of queueing behind it.
-    // tasks of a group: its tiles x the panel chunks
+    // One launch per shape, with its tiles x the panel chunks as tasks: long
+    // queries, then 32-row tiles, on the aux stream; 28- and 16-row tiles on
+    // the batch's stream.  A persistent kernel's CTAs that find no room start
+    // as another's leave, so the shapes of one stream fill the other's tail.
     const uint32_t nc = b->n_chunks;
-    const uint32_t n_long = b->n_long * nc, n_t32 = b->n_t32 * nc, n_t16 = b->n_t16 * nc;
     auto grid = [](int cap, uint32_t tasks) {
       return (int)std::max<uint64_t>(
           1, std::min<uint64_t>((uint64_t)cap, (tasks + kK2Warps - 1) / kK2Warps));
     };
-    const bool aux = n_long || n_t32;
-    const bool chk = b->sg_check;
+    const bool aux = b->n_tiles[kLongQuery] || b->n_tiles[kRows32];
+    // a group on the mode's second kernel; the f16 lanes have their own tables
+    auto second = [&](K2Params& T, bool on) {
+      if (!on || sc->mode != ESG_MODE_LOCAL) return on;
+      memcpy(T.tab_a, sc->tabh_a, sizeof T.tab_a);
+      memcpy(T.tab_b, sc->tabh_b, sizeof T.tab_b);
+      T.rec2 = half_pair(-sc->half_off);
+      T.bias = 0;
+      return on;
+    };
     if (aux) {
       ESG_CUDA(cudaEventRecord(sc->fork, st));
       ESG_CUDA(cudaStreamWaitEvent(sc->aux, sc->fork, 0));
     }
-    if (n_long) {
-      K2Params L = P;
-      L.n_tasks = n_long;
-      L.task_counter = b->d_counters + 3;
-      void* largs[] = {&L};
-      ESG_CUDA(cudaLaunchKernel(chk ? sc->k2c_long : sc->k2_long,
-                                dim3(grid(chk ? sc->blocksc_long : sc->blocks_long, n_long)),
-                                dim3(kK2Threads), largs, sc->k2_smem, sc->aux));
-      ++kernels;
-    }
-    if (n_t32) {
+    uint32_t tile0 = 0;
+    for (int k = 0; k < kShapes; tile0 += b->n_tiles[k], ++k) {
+      if (!b->n_tiles[k]) continue;
       K2Params T = P;
-      T.tasks = P.tasks + b->n_long;
-      T.n_tasks = n_t32;
-      T.task_counter = b->d_counters + 4;
+      T.tasks = P.tasks + tile0;
+      T.n_tasks = b->n_tiles[k] * nc;
+      static const int kCounter[kShapes] = {3, 4, 5, 0, 1 + 7};
+      T.task_counter = b->d_counters + kCounter[k];
+      const auto& kn = sc->k2[k][second(T, b->second[k])];
       void* targs[] = {&T};
-      ESG_CUDA(cudaLaunchKernel(chk ? sc->k2c_t32 : sc->k2_t32,
-                                dim3(grid(chk ? sc->blocksc_t32 : sc->blocks_t32, n_t32)),
-                                dim3(kK2Threads),
-                                targs, sc->k2_smem, sc->aux));
-      ++kernels;
-    }
-    if (n_t16) {
-      K2Params T = P;
-      T.tasks = P.tasks + b->n_long + b->n_t32;
-      T.n_tasks = n_t16;
-      T.task_counter = b->d_counters + 0;
-      void* targs[] = {&T};
-      ESG_CUDA(cudaLaunchKernel(chk ? sc->k2c_t16 : sc->k2_t16,
-                                dim3(grid(chk ? sc->blocksc_t16 : sc->blocks_t16, n_t16)),
-                                dim3(kK2Threads),
-                                targs, sc->k2_smem, st));
+      ESG_CUDA(cudaLaunchKernel(kn.fn, dim3(grid(kn.blocks, T.n_tasks)), dim3(kK2Threads), targs,
+                                sc->k2_smem, k == kLongQuery || k == kRows32 ? sc->aux : st));
       ++kernels;
     }
     if (aux) {
       ESG_CUDA(cudaEventRecord(sc->join, sc->aux));
       ESG_CUDA(cudaStreamWaitEvent(st, sc->join, 0));
     }
-    if (nc > 1) {
+    if (nc > 1 && !fused) {
       KMParams M{};
       M.order = b->d_order;
       M.n_order = b->n_order;
@@ -1544,7 +1623,7 @@ static esg_status launch_device_work(esg_scorer* sc, esg_batch* b, cudaStream_t 
       M.redo_base = b->host_list;
       M.redo_cap = b->redo_cap;
       const int blocks =
-          (int)std::max<uint64_t>(1, std::min<uint64_t>(4096, (b->n_order + 127) / 128));
+          (int)std::max<uint64_t>(1, std::min<uint64_t>(4096, (b->n_order + 3) / 4));
       void* margs[] = {&M};
       ESG_CUDA(cudaLaunchKernel((const void*)k2_merge_chunks, dim3(blocks), dim3(128), margs, 0,
                                 st));
@@ -1616,9 +1695,17 @@ static esg_status launch_device_work(esg_scorer* sc, esg_batch* b, cudaStream_t 
     M.ties = b->d_ties;
     M.rows = b->d_rows;
     M.n_refs = sc->n_refs;
-    const int blocks = (int)std::min<uint64_t>(4096, (b->n_reads + 255) / 256);
-    void* margs[] = {&M};
-    ESG_CUDA(cudaLaunchKernel((const void*)k5_merge, dim3(blocks), dim3(256), margs, 0, st));
+    if (fused) {
+      K5ChunkParams C{M, b->n_chunks, b->d_part_head, b->d_part_ties};
+      const int blocks = (int)std::min<uint64_t>(4096, (b->n_reads + 3) / 4);
+      void* cargs[] = {&C};
+      ESG_CUDA(cudaLaunchKernel((const void*)k5_merge_chunks, dim3(blocks), dim3(128), cargs, 0,
+                                st));
+    } else {
+      const int blocks = (int)std::min<uint64_t>(4096, (b->n_reads + 255) / 256);
+      void* margs[] = {&M};
+      ESG_CUDA(cudaLaunchKernel((const void*)k5_merge, dim3(blocks), dim3(256), margs, 0, st));
+    }
     ++kernels;
   }
   if (b->paired && b->n_pairs) {
@@ -1649,10 +1736,12 @@ static esg_status launch_device_work(esg_scorer* sc, esg_batch* b, cudaStream_t 
 static uint32_t work_key(const esg_scorer* sc, const esg_batch* b) {
   const uint32_t nc = b->n_chunks;
   const bool k3 = b->host_list + b->redo_cap > 0;
-  return (b->n_long ? 1u : 0u) | (b->n_t32 ? 2u : 0u) | (b->n_t16 ? 4u : 0u) |
-         ((b->n_tasks && nc > 1) ? 8u : 0u) | (k3 ? 16u : 0u) | (b->n_reads ? 32u : 0u) |
-         ((b->paired && b->n_pairs) ? 64u : 0u) | (b->sg_check ? 128u : 0u) |
-         (b->kernel == ESG_KERNEL_PLAIN32 ? 256u : 0u) | (sc->mode == ESG_MODE_LOCAL ? 512u : 0u);
+  uint32_t key = ((b->n_tasks && nc > 1) ? 1u : 0u) | (k3 ? 2u : 0u) | (b->n_reads ? 4u : 0u) |
+                 ((b->paired && b->n_pairs) ? 8u : 0u) |
+                 (b->kernel == ESG_KERNEL_PLAIN32 ? 16u : 0u) | (fused_merge(b) ? 32u : 0u);
+  for (int k = 0; k < kShapes; ++k)
+    key |= (b->n_tiles[k] ? 1u : 0u) << (8 + 2 * k) | (b->second[k] ? 1u : 0u) << (9 + 2 * k);
+  return key;
 }
 
 // The batch's device work as one CUDA graph launch on `st`: the launch
@@ -1733,12 +1822,12 @@ esg_status esg_submit(esg_scorer* sc, esg_batch* b) {
   b->d_tasks = carve<uint2>(at, b->n_tasks ? b->n_tasks : 1);
   b->d_list = carve<uint32_t>(at, nlist ? nlist : 1);
   b->d_chunks = carve<uint32_t>(at, b->n_chunks + 1);
-  b->d_counters = carve<uint32_t>(at, 8);
   b->d_qhead = carve<int4>(at, nq);
   b->d_qties = carve<uint32_t>(at, nq * sc->cap);
   b->d_k3out = carve<int32_t>(at, nlist ? (size_t)nlist * sc->n_refs : 1);
   b->d_results = carve<int4>(at, nr);
   b->d_ties = carve<uint32_t>(at, nr * sc->cap);
+  b->d_counters = carve<uint32_t>(at, kCounters);
   b->d_rows = dev_rows ? carve<int32_t>(at, nq * sc->n_refs) : nullptr;
   b->d_pairs = np ? carve<int4>(at, 2 * np) : nullptr;
   b->d_pties = np ? carve<uint32_t>(at, np * sc->cap) : nullptr;
@@ -1784,11 +1873,11 @@ esg_status esg_submit(esg_scorer* sc, esg_batch* b) {
   b->h_rows = rows ? carve<int32_t>(o, nq * sc->n_refs) : nullptr;
   b->h_pairs = np ? carve<int4>(o, 2 * np) : nullptr;
   b->h_pties = np ? carve<uint32_t>(o, np * sc->cap) : nullptr;
-  // d_results and d_ties are adjacent in device memory, as in the staging
+  // d_results, d_ties and d_counters are adjacent in device memory, as in the
+  // staging
   ESG_CUDA(cudaMemcpyAsync(b->h_results, b->d_results,
-                           carve_size(nr, 16) + carve_size(nr * sc->cap, 4),
+                           carve_size(nr, 16) + carve_size(nr * sc->cap, 4) + 16,
                            cudaMemcpyDeviceToHost, st));
-  ESG_CUDA(cudaMemcpyAsync(b->h_counters, b->d_counters, 16, cudaMemcpyDeviceToHost, st));
   if (rows)
     ESG_CUDA(cudaMemcpyAsync(b->h_rows, b->d_rows, (size_t)b->n_q * sc->n_refs * 4,
                              cudaMemcpyDeviceToHost, st));

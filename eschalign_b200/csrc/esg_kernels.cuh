@@ -3,19 +3,18 @@
 // Four kernels, launched in this order on one stream per batch:
 //
 //   k2_batched   the product: every (query, reference pair) of the panel in
-//                int16x2 lanes.  One warp is a 32-lane systolic array: each
-//                lane holds a 16- or 32-row stripe of one query (G, E and
-//                the row's substitution table or score-record address in
+//                16-bit lanes.  One warp is a 32-lane systolic array: each
+//                lane holds a 16-, 28- or 32-row stripe of one query (two
+//                state words and the row's score-record address in
 //                registers) and walks the columns of a reference pair; the
 //                stripe's bottom row goes to the next lane by shuffle, so no
 //                DP state ever leaves the register file.  The two 16-bit
 //                halves of every register are two references (a
-//                length-sorted pair).  Substitution is one PRMT per cell
-//                pair, or (local mode, and semi-global 32-row stripes) one
-//                shared-memory load from the lane's per-column score record;
-//                the recurrence is three VIADDMNMX and one VIMNMX (DPX) plus
-//                one IMAD.  The argmax / tie / XS reduction is folded in per
-//                query, online, in shared memory.
+//                length-sorted pair).  Substitution is one shared-memory load
+//                from the lane's per-column score record; the recurrence is
+//                three DPX instructions plus two adds on the FMA pipe.  The
+//                argmax / tie / XS reduction is folded in per query, online,
+//                in shared memory.
 //                Pairs that may have left int16 are flagged and their query
 //                is re-scored by the int32 kernel.
 //   k3_lanes     the exact int32 path: the recurrence of
@@ -26,7 +25,8 @@
 //                pair comparison arm.
 //   k4_rows      per-query reduction of k3's rows (mapper.rs:444-472).
 //   k5_merge     per read: forward and reverse-complement query states
-//                merged into the read's result.
+//                merged into the read's result (k5_merge_chunks: straight
+//                from the panel chunks' states).
 //   k6_pairs     paired batches: per pair, the (reference, template strand)
 //                candidates of crates/eschalign/src/mapper/pair.rs:195-234
 //                ranked from the four mate rows (one warp per pair).
@@ -43,27 +43,12 @@ constexpr int kBiasLocal = 2048;      // local: H + B >= B >= |o|, |e|
 constexpr int kBiasSemiGlobal = -16384;  // semi-global: H + B < 0 while |H| < 12000
 constexpr int kNeg32 = -(1 << 29);    // int32 stand-in for -infinity, i32::MIN / 4 (scalar.rs:42)
 // k2 CTA shape: 4 warps, 4 resident CTAs per SM (16 warps, <= 128
-// registers; 3 for 32-row stripes).  Tuning knobs, each measured on B200 on
-// the C2 workload (1 M reads of ~110 nt x 164 references, both strands):
+// registers; 3 for 28- and 32-row stripes).  Measured on B200 on the C2
+// workload (reads of ~110 nt x 164 references, both strands):
 //   ESG_K2_WARPS / ESG_K2_MIN_BLOCKS  CTA shape (4 x 4 beat 4 x 5 at 96
-//       registers once local mode reads its scores from shared memory, and
-//       8 warps x 2 CTAs)
-//   ESG_SC_LDS  modes whose per-cell scores come from a per-thread record in
-//       shared memory (bit 0 local, bit 1 semi-global) instead of one PRMT
-//       per cell: local +5.0 %; semi-global on 32-row stripes
-//       (ESG_SC_LDS_SG_MINR 32) +1.9 % on C4 pairs and C2 semi-global once
-//       its last-column snapshot stopped spilling (-1.0 % before), 16-row
-//       stripes as well -0.4 %
-//   ESG_SEL_PREFETCH  modes that load a lane's next column selector a column
-//       ahead (bit 0 local, bit 1 semi-global): +2 % in both with the above
-//   ESG_STEADY_UNROLL  unroll of local mode's unchecked column loop, 16-row
-//       stripes (8: +0.9 % over 4)
-//   ESG_STEADY_UNROLL32  the same for 32-row stripes reading the panel from
-//       L2 (C3: 4 +3.9 % over 1, 8 -1.1 % against 4); with the panel in
-//       shared memory they stay at 1 (unrolled, they spill)
-//   ESG_K2_R32_BLOCKS  resident CTAs of 32-row stripes (3; 2 lets
-//       semi-global keep its state without spilling but measured -4.6 % on
-//       C2 semi-global, local and C3 unchanged)
+//       registers, and 8 warps x 2 CTAs)
+//   ESG_K2_R32_BLOCKS  resident CTAs of 28- and 32-row stripes (3; at 4 they
+//       spill 124-212 bytes and lose 2-5 %, at 2 -4.6 %)
 #ifndef ESG_K2_WARPS
 #define ESG_K2_WARPS 4
 #endif
@@ -73,18 +58,6 @@ constexpr int kNeg32 = -(1 << 29);    // int32 stand-in for -infinity, i32::MIN 
 #ifndef ESG_K2_R32_BLOCKS
 #define ESG_K2_R32_BLOCKS 3
 #endif
-#ifndef ESG_SC_LDS
-#define ESG_SC_LDS 3
-#endif
-#ifndef ESG_SEL_PREFETCH
-#define ESG_SEL_PREFETCH 3
-#endif
-#ifndef ESG_STEADY_UNROLL
-#define ESG_STEADY_UNROLL 8
-#endif
-#ifndef ESG_STEADY_UNROLL32
-#define ESG_STEADY_UNROLL32 4
-#endif
 constexpr int kK2Warps = ESG_K2_WARPS;  // warps per k2 CTA
 constexpr int kK2Threads = kK2Warps * 32;
 constexpr uint32_t kFull = 0xffffffffu;
@@ -92,18 +65,31 @@ constexpr uint32_t kNoRef = 0xffffffffu;
 constexpr uint32_t kMaxCap = 32;       // largest tie capacity (ESG_MAX_TIE_CAPACITY)
 // per-thread shared words of the column score record (one per row code
 // 0-5), word c of thread t at c * kK2Threads + t: every thread in its own bank
-constexpr int kScrWords = ESG_SC_LDS ? 6 : 0;
+constexpr int kScrWords = 6;
 constexpr uint32_t kScrStride = (uint32_t)kK2Threads * 4;  // bytes between code words
-#ifndef ESG_SC_LDS_SG_MINR
-#define ESG_SC_LDS_SG_MINR 32
-#endif
-template <bool kLocal, int R>
-__host__ __device__ constexpr bool sc_lds() {
-  return (ESG_SC_LDS & (kLocal ? 1 : 2)) != 0 && (kLocal || R >= ESG_SC_LDS_SG_MINR);
-}
-template <bool kLocal>
-__host__ __device__ constexpr bool sel_prefetch() {
-  return (ESG_SEL_PREFETCH & (kLocal ? 1 : 2)) != 0;
+// What the 16-bit halves of k2's registers hold (see pair_pass).
+enum K2Lanes {
+  kLanesInt,      // biased int16
+  kLanesChecked,  // the same, semi-global, every cell watched for an overflow
+  kLanesHalf,     // local: unbiased whole numbers 0..2047 as f16 subnormals
+};
+constexpr int kHalfMax = 2047;           // largest score kLanesHalf holds exactly
+constexpr uint32_t kHalfOne = 0x3c003c00u;  // 1.0 in both halves
+// Unroll of k2's unchecked column loop.  Unrolled once, the loop spends up to
+// 1.4 register moves a cell pair (of 7.9 instructions) on the rotated state;
+// unrolled past about 16 KB of code it outruns the instruction cache.  Swept
+// 1-8 on B200, 150 000 C2 reads on one shape: local f16, 32 rows 133 / 121 /
+// 125 / 122 ms at 1 / 2 / 3 / 4; semi-global, 32 rows 129 / 120 / 126 at 2 /
+// 3 / 4; reading the panel through L2, semi-global 205 at 3, 197 at 6; int16
+// local 28 + 32 rows 138 / 128 / 130 at 1 / 2 / 3; long queries 53.5 / 63 /
+// 80 at 2 / 4 / 6 (two stripe heights share the cache).
+template <int R, bool kSmem, bool kLong>
+__host__ __device__ constexpr int steady_unroll(bool local, int lanes) {
+  if (kLong) return 2;
+  if (R == 8) return 4;
+  if (lanes == kLanesHalf) return R == 16 ? 3 : kSmem ? 2 : 4;
+  if (!local) return R == 16 || kSmem ? 3 : 6;
+  return R == 16 ? 8 : kSmem ? 2 : 4;
 }
 
 // error bits in counters[2]
@@ -139,6 +125,23 @@ __device__ __forceinline__ uint32_t mad_lo(uint32_t a, uint32_t b, uint32_t c) {
   uint32_t d;
   asm("mad.lo.u32 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(c));
   return d;
+}
+// max(a + b, 0) and a + b per f16 half, on the FMA pipe.  Whole numbers n
+// with |n| <= 2047 are kept as n * 2^-24 (sign and magnitude n; exact sums),
+// so a result >= 0 is the integer n itself to the integer min / max ops.
+__device__ __forceinline__ uint32_t add_relu_f16x2(uint32_t a, uint32_t b) {
+  uint32_t d;
+  asm("fma.rn.relu.f16x2 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(kHalfOne), "r"(b));
+  return d;
+}
+__device__ __forceinline__ uint32_t add_f16x2(uint32_t a, uint32_t b) {
+  uint32_t d;
+  asm("add.rn.f16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
+  return d;
+}
+// the whole number n (|n| <= 1023) as a pair of f16 subnormals
+__host__ __device__ __forceinline__ uint32_t half_pair(int n) {
+  return (n < 0 ? 0x8000u | (uint32_t)(-n) : (uint32_t)n) * 0x10001u;
 }
 __device__ __forceinline__ uint32_t max16x2(uint32_t a, uint32_t b) {
   uint32_t d;
@@ -219,6 +222,8 @@ struct K2Params {
   // scoring, pre-shifted by the gap open (see k2_batched)
   uint32_t tab_a[6];
   uint32_t tab_b[6];
+  uint32_t rec2;         // kLanesHalf: added to a table's score to give s (see pair_pass)
+  int32_t borrow;        // semi-global: some s - o is negative
   uint32_t e2;           // e in both halves
   int32_t o, e;
   int32_t bias;          // value bias of the int16 lanes
@@ -288,47 +293,51 @@ __device__ __forceinline__ bool stage_panel(void* smem, const void* gsrc, uint32
   return __syncthreads_and(ok) != 0;
 }
 
-// One systolic pass of a warp over the columns of one reference pair.
+// One systolic pass of a warp over the columns of one reference pair, two
+// references per register (low half: the longer one of the pair, high half:
+// the shorter one).
 //
-// Values are held biased: every H, E, F of the recurrence is stored as
-// value + B (B = bias: +2048 in local mode, -16384 in semi-global), in signed
-// 16-bit halves, two references per register (low half: the longer
-// reference of the pair, high half: the shorter one).
+// What bounds it is the integer ALU (every DPX instruction, PRMT and plain
+// MAX takes the same 64-lane-a-clock issue port; the FMA pipe beside it is
+// as wide), and behind it the F chain down a stripe's rows (three dependent
+// instructions a row), which 12-16 warps an SM hide.  So a cell pair is
+// written for the fewest ALU instructions -- E, F and H, one DPX instruction
+// each, and half a VIMNMX3 for the running best where there is one -- with
+// both remaining adds (the diagonal term, G = H + open) on the FMA pipe:
 //
-// Lane state (rows r = 0..15 of the lane's stripe):
-//   ta[r], tb[r]  PRMT tables of the row's read code c (or, with score
-//                 records, the shared address of code c's word): byte x of {tb, ta} is
-//                 s(c, x) - o for reference code x = 0..3, 4 (wildcard), and
-//                 a padding column's score at x = 5.  Both halves use the
-//                 same table; the column's selector picks a byte per half
-//                 and sign-extends it to 16 bits.
-//   g[r]          G = H + o + B of the row at the previous column
-//   ev[r]         E + B of the row at the previous column
-// Every integer ALU instruction (PRMT, the DPX VIADDMNMX / VIMNMX3, plain
-// MAX) takes the same ALU issue slot, so the loop is written for the fewest
-// of them: G feeds E of the next column and F of the next row (one
-// VIADDMNMX each: max(X + e, G)); the diagonal term is G_diag + (s - o), which
-// is why the tables hold s - o (one VIADDMNMX); H + B = max(h1, F, B) is one
-// VIMNMX3 in local mode (B, the zero floor), one MAX in semi-global; the
-// running best takes one VIMNMX3 per two rows.  G = H + B + o is a 32-bit
-// IMAD (H * 1 + o * 65537, on the FMA pipe): exact in both halves because
-// the low half's value is never in [0, |o|) -- local H + B >= B >= |o|,
-// semi-global H + B < 0 -- so its borrow cancels the constant's, and the
-// high half's carry-out is discarded.  Padding columns (garbage that may
-// wrap) are only ever in the high half.  5.5 ALU instructions per cell pair
-// in local mode, 5 in semi-global, plus one IMAD.
+//   kLanesHalf (local, scores up to 2047)  Halves hold H, E, F >= 0 as whole
+//     numbers, which are also the f16 subnormals n * 2^-24: sums of those are
+//     exact and HFMA2.relu gives max(a + b, 0), the local floor, for free.
+//     d = relu(H_diag + s), H = max3(d, E, F), G = relu(H + o),
+//     E = max(E + e, G), F = max(F + e, G).  E and F floored at 0 change no H
+//     (the floor is 0).  3.5 ALU.  g[r] holds d of the row's next column (its
+//     record is written a column ahead), so that nothing old outlives the
+//     update and the registers need no rotation.  The best is taken over d:
+//     E and F never exceed an earlier H.
+//   kLanesInt, semi-global  Halves hold value + B (B = -16384) in int16;
+//     g[r] = G = H + o + B of the row at the previous column.
+//     d = G_diag + (s - o) and G = H + o are 32-bit IMADs, exact in both
+//     halves: the low half's sums stay negative (static bound, or watched, see
+//     kLanesChecked), so a negative addend's carry out is the rule, cancelled
+//     by o * 65537 or by a record word built with one less above it
+//     (P.borrow), and the high half's carry is discarded.  Padding columns
+//     (garbage that may wrap) are only ever in the high half.  3 ALU.
+//   kLanesInt, local  B = 2048; d takes the ALU (max(G_diag + (s - o), E)) as
+//     nothing else gives the floor.  4.5 ALU.  For scores past 2047.
 //
-// Score records (kLds, local mode): the PRMT moves from every cell to every
-// column.  At each column the lane writes the column's score word for each
-// read code (PRMT of that code's tables, codes 0-3, and the wildcard code 4
-// when the warp holds a wildcard row) to its own record in shared memory,
-// then each row loads its code's word: ta[r] holds that word's shared
-// address instead of a table.  The padding code's word is a constant written
-// once per pass (local: -128 in both halves, H stays 0 under the floor).
-// The record's words of one code are kK2Threads words apart, so every lane
-// reads and writes its own bank.  4.5 ALU instructions per cell pair plus
-// four PRMTs per column, one shared load per cell pair, one IMAD; the
-// loads go to the otherwise idle load/store pipe (C2 local: +5 %).
+// C2 local, 150 000 reads: 115.8 ms; with 4.5 ALU on 16-row stripes (the best
+// of before) 137.5.  Semi-global 115.7 against 130.7 (5 ALU, 32 rows).
+//
+// Score records: at each column the lane writes the column's score word for
+// each read code (PRMT of that code's tables by the column's selector, which
+// picks a byte per half and sign-extends it; codes 0-3, and the wildcard code
+// 4 when the warp holds a wildcard row) to its own record in shared memory,
+// then each row loads its code's word: ta[r] is that word's address.  Tables
+// {tb, ta}: byte x is s(c, x) - o for reference code x = 0..3, 4 (wildcard),
+// and a padding column's score at x = 5; for kLanesHalf s + off (0..127, off
+// taken off again by P.rec2, padding columns 0).  The padding code's word is a
+// constant.  The words of one code are kK2Threads apart, so every lane reads
+// and writes its own bank.
 //
 // The lane with skew k works on column j = t - k at step t; its top input
 // (G and F of the row above) is the previous lane's bottom output of step
@@ -340,7 +349,7 @@ __device__ __forceinline__ bool stage_panel(void* smem, const void* gsrc, uint32
 //
 // Returns, per lane, the pass's local best (H + B) or semi-global last-column
 // maximum (G, the short half's taken at its own end) in `v`, and the
-// semi-global maximum of row 15 over the lane's columns (H + B) in `lr`.
+// semi-global maximum of the last row over the lane's columns (H + B) in `lr`.
 struct PassConst {
   uint32_t g0, neg2, e2, o32, one, bias2;
 };
@@ -359,23 +368,27 @@ __device__ __forceinline__ uint32_t load_sel(const uint16_t* sp, int j) {
   }
 }
 
-template <int R, bool kLocal, bool kPanelW, bool kLong, bool kSmem, bool kCheck>
+template <int V>
+struct IntConst {
+  static constexpr int value = V;
+};
+
+template <int R, bool kLocal, bool kLong, bool kSmem, int kLanes>
 __device__ __forceinline__ void pair_pass(const K2Params& P, uint32_t scr, bool wild,
-                                          const uint32_t (&ta)[R],
-                                          const uint32_t (&tb)[kPanelW ? R : 1], int skew,
+                                          const uint32_t (&ta)[R], int skew,
                                           bool active_lane, bool first, uint32_t padmask, int m,
                                           int jshort, const uint16_t* __restrict__ sp, int steps,
                                           const PassConst& K, uint2* buf, bool from_buf,
                                           bool to_buf, uint32_t& v, uint32_t& lr, uint32_t& am) {
   const int lane = threadIdx.x & 31;
-  constexpr bool kLds = sc_lds<kLocal, R>() && !kLong;
-  constexpr bool kPre = sel_prefetch<kLocal>();
-  if constexpr (kLds) {
-    // padding rows: local, -128 against every column (H stays 0 under the
-    // floor); semi-global, s = 0 (H = 0 exactly against real columns; the
-    // short half's columns past its end are never read)
-    st_shared_u32(scr + 5 * kScrStride, kLocal ? 0xff80ff80u : pack16x2(-P.o, -P.o));
-  }
+  constexpr bool kCheck = kLanes == kLanesChecked;
+  constexpr bool kHalf = kLanes == kLanesHalf;
+  constexpr bool kPre = kLocal && (kSmem || !kHalf);
+  // padding rows: local, -128 (kLanesHalf: 0) against every column, so H
+  // stays 0 under the floor; semi-global, s = 0 (H = 0 exactly against real
+  // columns; the short half's columns past its end are never read)
+  st_shared_u32(scr + 5 * kScrStride,
+                kHalf ? 0u : kLocal ? 0xff80ff80u : pack16x2(-P.o, -P.o));
   uint32_t g[R], ev[R];
 #pragma unroll
   for (int r = 0; r < R; ++r) {
@@ -387,70 +400,112 @@ __device__ __forceinline__ void pair_pass(const K2Params& P, uint32_t scr, bool 
   // local: max H + B over this lane's cells; checked semi-global: the same
   // without the floor (the short half's taken at its own end)
   uint32_t best = kLocal ? K.bias2 : K.neg2, s_best = K.neg2;
-  uint32_t lastrow = K.neg2;               // semi-global: max H + B of row 15
+  uint32_t lastrow = K.neg2;               // semi-global: max H + B of the last row
   uint32_t s_col = K.neg2, s_last = K.neg2;  // semi-global short-half snapshot
   // inactive lanes of a tile sit at a skew no step reaches; only the long
   // path needs the per-lane bound (its lanes past the query's last stripe)
   const int mlim = (kLong && !active_lane) ? 0 : m;
+  // (kPre: +2 % where the panel is in shared memory)
   uint32_t seln = kPre ? load_sel<kSmem>(sp, 0) : 0u;
 
+  // a column's score record: one word per read code, in this thread's own
+  // bank, read back per row (wildcard rows only when the warp has some)
+  auto record = [&](uint32_t sel) {
+    auto word = [&](int c) {
+      uint32_t w = prmt(P.tab_a[c], P.tab_b[c], sel);
+      if constexpr (kHalf) w = add_f16x2(w, P.rec2);
+      if constexpr (!kLocal)
+        if (P.borrow) w -= (w << 1) & 0x10000u;
+      st_shared_u32(scr + c * kScrStride, w);
+    };
+#pragma unroll
+    for (int c = 0; c < 4; ++c) word(c);
+    if (wild) word(4);
+  };
+  if constexpr (kHalf) {
+    // column 0's diagonal terms, from the zero border
+    record(kPre ? seln : load_sel<kSmem>(sp, 0));
+#pragma unroll
+    for (int r = 0; r < R; ++r) g[r] = add_relu_f16x2(K.g0, ld_shared_u32(ta[r]));
+    if constexpr (kPre) seln = load_sel<kSmem>(sp, 1);
+  }
+  uint2 bnext = make_uint2(0u, 0u);
+  if constexpr (kLong)
+    if (from_buf && lane == 0) bnext = buf[0];
   // One column of the lane's stripe, given the top input (G, F of the row
   // above at this column).
-  auto column = [&](int j, uint32_t gt, uint32_t ft) {
+  auto column = [&](auto snap, int j, uint32_t gt, uint32_t ft) {
+    constexpr bool kSnap = decltype(snap)::value != 0;
     if constexpr (kLong) {
       if (from_buf && lane == 0) {
-        const uint2 b = buf[j];
-        gt = b.x;
-        ft = b.y;
+        gt = bnext.x;
+        ft = bnext.y;
+        bnext = buf[min(j + 1, m - 1)];  // a column ahead: its latency is off the chain
       }
     }
+    // columns of a lane come in order: with kPre the next one's selector is
+    // loaded a column ahead
+    constexpr int kAhead = kHalf ? 1 : 0;
     uint32_t sel;
     if constexpr (kPre) {
-      // columns of a lane come in order: the next one's selector is loaded
-      // a column ahead (the blob holds one spare selector past the last pair)
       sel = seln;
-      seln = load_sel<kSmem>(sp, j + 1);
+      seln = load_sel<kSmem>(sp, j + kAhead + 1);
     } else {
-      sel = load_sel<kSmem>(sp, j);
+      sel = load_sel<kSmem>(sp, j + kAhead);
     }
-    if constexpr (kLds) {
-      // the column's score record: one word per read code, in this thread's
-      // own bank, read back per row below (wildcard rows only when the warp
-      // has some)
+    record(sel);
+    if constexpr (kHalf) {
+      uint32_t f = ft, up = gt, prev = 0;
 #pragma unroll
-      for (int c = 0; c < 4; ++c) st_shared_u32(scr + c * kScrStride, prmt(P.tab_a[c], P.tab_b[c], sel));
-      if (wild) st_shared_u32(scr + 4 * kScrStride, prmt(P.tab_a[4], P.tab_b[4], sel));
+      for (int r = 0; r < R; ++r) {
+        const uint32_t d = g[r];
+        const uint32_t h = __vimax3_s16x2(d, ev[r], f);
+        if (r & 1)
+          best = __vimax3_s16x2(best, prev, d);
+        else
+          prev = d;
+        g[r] = add_relu_f16x2(up, ld_shared_u32(ta[r]));
+        const uint32_t gr = add_relu_f16x2(h, K.o32);
+        ev[r] = __viaddmax_s16x2(ev[r], K.e2, gr);
+        f = __viaddmax_s16x2(f, K.e2, gr);
+        up = h;
+      }
+      gbot = up;
+      fbot = f;
+      if constexpr (kLong) {
+        if (to_buf && lane == 31) buf[j] = make_uint2(gbot, fbot);
+      }
+      return;
     }
-    uint32_t gd = gdc;
+    uint32_t gup = gt, f = ft, h15 = 0, hprev = 0, gd = gdc;
     gdc = gt;
-    uint32_t gup = gt, f = ft, h15 = 0, hprev = 0;
+    // semi-global: a row's diagonal term is taken before the row above
+    // overwrites the G it reads, which lets every g[r] stay in its register
+    auto diag = [&](int r) {
+      return mad_lo(r ? g[r ? r - 1 : 0] : gd, K.one, ld_shared_u32(ta[r]));
+    };
+    uint32_t dn = kLocal ? 0u : diag(0);
 #pragma unroll
     for (int r = 0; r < R; ++r) {
-      uint32_t sc;
-      if constexpr (kLds)
-        sc = ld_shared_u32(ta[r]);
-      else
-        sc = prmt(ta[r], tb[kPanelW ? r : 0], sel);
+      const uint32_t d = dn;
+      if constexpr (!kLocal)
+        if (r + 1 < R) dn = diag(r + 1 < R ? r + 1 : r);
       ev[r] = __viaddmax_s16x2(ev[r], K.e2, g[r]);
       f = __viaddmax_s16x2(f, K.e2, gup);
-      const uint32_t h1 = __viaddmax_s16x2(gd, sc, ev[r]);
       uint32_t h;
       if constexpr (kLocal) {
+        const uint32_t h1 = __viaddmax_s16x2(gd, ld_shared_u32(ta[r]), ev[r]);
+        gd = g[r];
         h = __vimax3_s16x2(h1, f, K.bias2);
+      } else {
+        h = __vimax3_s16x2(d, ev[r], f);
+      }
+      if constexpr (kLocal || kCheck) {
         if (r & 1)
           best = __vimax3_s16x2(best, hprev, h);
         else
           hprev = h;
-      } else {
-        h = max16x2(h1, f);
-        if constexpr (kCheck) {
-          if (r & 1)
-            best = __vimax3_s16x2(best, hprev, h);
-          else
-            hprev = h;
-        }
       }
-      gd = g[r];
       g[r] = mad_lo(h, K.one, K.o32);
       gup = g[r];
       if (r == R - 1) h15 = h;
@@ -462,7 +517,7 @@ __device__ __forceinline__ void pair_pass(const K2Params& P, uint32_t scr, bool 
     }
     if constexpr (!kLocal) {
       lastrow = max16x2(lastrow, h15);
-      if (j == jshort) {
+      if (kSnap && j == jshort) {
         // the short half's last column, padding rows left out.  Padding
         // rows hold G = o + B exactly (H = 0), so a maximum above that is a
         // read row's and the unmasked maximum stands; only a maximum equal
@@ -495,37 +550,31 @@ __device__ __forceinline__ void pair_pass(const K2Params& P, uint32_t scr, bool 
   };
 
   int t = 0;
-  // (local mode only: semi-global measured slower with a second copy of the
-  // column body, whose last-row and short-reference state cost it registers:
-  // again at 4 CTAs and 128 registers, -0.7 % to -1.6 % for unrolls 1-8 on
-  // C2 semi-global, its 32-row stripes spilling more; and once the snapshot
-  // stopped spilling, on 32-row stripes alone, -2.0 % on C4 pairs)
-  if constexpr (kLocal && !kLong) {
-    // Steps fill .. m - 1, where fill = steps - m is the tile's largest skew,
-    // have every lane of the tile's queries inside the pair's columns: they
-    // run without the column check.  Lanes past the tile's queries take
-    // skew 0 there (columns in range, values nobody reads: only later lanes,
-    // also past the queries, see them, and a pass's results are taken from
-    // the queries' own lanes).
-    const int fill = steps - m;
-    if (fill < m) {
+  // Steps fill .. m - 1, where fill = steps - m is the largest skew, have
+  // every lane of the task's queries inside the pair's columns: they run
+  // without the column check, and in semi-global mode (up to the first lane's
+  // snapshot column) without the snapshot, whose code would fill the
+  // instruction cache.  Lanes past the queries take skew 0 there (columns in
+  // range, values nobody reads: only later lanes, also past the queries, see
+  // them, and a pass's results are taken from the queries' own lanes; a long
+  // query's local best takes padding rows in too, which add nothing to H).
+  const int fill = steps - m;
+  const int full = (kLocal || jshort < 0) ? m : jshort;
+  if (fill < full) {
 #pragma unroll 1
-      for (; t < fill; ++t) {
-        uint32_t gt, ft;
-        top(gt, ft);
-        const int j = t - skew;
-        if ((unsigned)j < (unsigned)mlim) column(j, gt, ft);
-      }
-      const int sk = active_lane ? skew : 0;
-      // unrolled (ESG_STEADY_UNROLL, ESG_STEADY_UNROLL32); 32-row stripes
-      // with the panel in shared memory have no registers to spare
-      constexpr int kUnroll = R <= 16 ? ESG_STEADY_UNROLL : (kSmem ? 1 : ESG_STEADY_UNROLL32);
+    for (; t < fill; ++t) {
+      uint32_t gt, ft;
+      top(gt, ft);
+      const int j = t - skew;
+      if ((unsigned)j < (unsigned)mlim) column(IntConst<0>{}, j, gt, ft);
+    }
+    const int sk = active_lane ? skew : 0;
+    constexpr int kUnroll = steady_unroll<R, kSmem, kLong>(kLocal, kLanes);
 #pragma unroll kUnroll
-      for (; t < m; ++t) {
-        uint32_t gt, ft;
-        top(gt, ft);
-        column(t - sk, gt, ft);
-      }
+    for (; t < full; ++t) {
+      uint32_t gt, ft;
+      top(gt, ft);
+      column(IntConst<0>{}, t - sk, gt, ft);
     }
   }
 #pragma unroll 1
@@ -533,7 +582,7 @@ __device__ __forceinline__ void pair_pass(const K2Params& P, uint32_t scr, bool 
     uint32_t gt, ft;
     top(gt, ft);
     const int j = t - skew;
-    if ((unsigned)j < (unsigned)mlim) column(j, gt, ft);
+    if ((unsigned)j < (unsigned)mlim) column(IntConst<1>{}, j, gt, ft);
   }
   am = K.neg2;
   if constexpr (kLocal) {
@@ -555,13 +604,12 @@ __device__ __forceinline__ void pair_pass(const K2Params& P, uint32_t scr, bool 
   }
 }
 
-// Row tables of stripe `s` of a query (n codes at q, reverse complement if
-// rc): row r is read row i = 16 s + r - pad; rows before the read are padding.
-template <int R, bool kPanelW, bool kLds>
-__device__ __forceinline__ bool row_tables(const K2Params& P, const uint8_t* q, uint32_t n,
-                                           bool rc, bool valid, int s, int pad,
-                                           uint32_t (&ta)[R],
-                                           uint32_t (&tb)[kPanelW ? R : 1], uint32_t scr = 0) {
+// Record addresses of stripe `s` of a query (n codes at q, reverse complement
+// if rc): row r is read row i = R s + r - pad; rows before the read are
+// padding.  Returns whether any lane of the warp has a wildcard row.
+template <int R>
+__device__ __forceinline__ bool row_records(const uint8_t* q, uint32_t n, bool rc, bool valid,
+                                            int s, int pad, uint32_t scr, uint32_t (&ta)[R]) {
   bool wild = false;
 #pragma unroll
   for (int r = 0; r < R; ++r) {
@@ -573,14 +621,8 @@ __device__ __forceinline__ bool row_tables(const K2Params& P, const uint8_t* q, 
       c = (rc && x < 4) ? 3 - x : x;
     }
     wild |= c == 4;
-    if constexpr (kLds) {
-      ta[r] = scr + c * kScrStride;  // the row code's word in the column record
-    } else {
-      ta[r] = P.tab_a[c];
-      if constexpr (kPanelW) tb[r] = P.tab_b[c];
-    }
+    ta[r] = scr + c * kScrStride;  // the row code's word in the column record
   }
-  if constexpr (!kPanelW) tb[0] = P.tab_b[0];
   return __any_sync(kFull, wild);
 }
 
@@ -591,7 +633,7 @@ __device__ __forceinline__ bool row_tables(const K2Params& P, const uint8_t* q, 
 // H + B >= 0 (H >= 16384), where G's IMAD may borrow wrongly (see
 // pair_pass) -- the first such cell is itself exact, its inputs being below
 // the mark, so the maximum over every cell, `am`, catches it.
-template <bool kLocal, bool kCheck>
+template <bool kLocal, int kLanes>
 __device__ __forceinline__ void fold_pair(const K2Params& P, int* slot, uint32_t* sties,
                                           uint32_t cap, uint4 pm, int mB, bool rc, uint32_t qid,
                                           uint32_t v, uint32_t lr, uint32_t am, int bias) {
@@ -599,11 +641,12 @@ __device__ __forceinline__ void fold_pair(const K2Params& P, int* slot, uint32_t
   if constexpr (kLocal) {
     scA = lo16(v) - bias;
     scB = hi16(v) - bias;
-    if (scA >= P.sat || (mB > 0 && scB >= P.sat)) slot[3] |= kQRedo;
+    if constexpr (kLanes == kLanesInt)
+      if (scA >= P.sat || (mB > 0 && scB >= P.sat)) slot[3] |= kQRedo;
   } else {
     scA = max(lo16(v) - P.o, lo16(lr)) - bias;
     scB = max(hi16(v) - P.o, hi16(lr)) - bias;
-    if constexpr (kCheck)
+    if constexpr (kLanes == kLanesChecked)
       if (lo16(am) >= 0 || (mB > 0 && hi16(am) >= 0)) slot[3] |= kQRedo;
   }
   const uint32_t rbit = rc ? 1u : 0u;
@@ -640,20 +683,24 @@ __device__ __forceinline__ void flush_query(const K2Params& P, uint32_t qid, uin
   }
 }
 
-// One warp, one task at a time, tasks pulled from an atomic counter.  The
-// kernel is instantiated twice: kLong = false takes tiles of up to 32
-// queries whose stripes fill the warp's lanes (a query of n rows takes
-// S = ceil(n / 16) lanes), scored in one pass per reference pair; kLong =
-// true takes one long query (S > 32) per task, scored in ceil(S / 32) passes
-// per pair chained through a per-warp column buffer in global memory.  Two
-// instantiations keep the register allocation of the short-read path free of
-// the long path's state; the host runs them concurrently.
-// Stripes are aligned so the read's last row is row 15 of its last stripe;
-// the 16 S - n rows before the read's first row score 0 against every real
+// One warp, one task at a time, tasks pulled from an atomic counter.
+// kLong = false takes tiles of up to 32 queries whose stripes fill the warp's
+// lanes (a query of n rows takes S = ceil(n / R) lanes), scored in one pass
+// per reference pair; kLong = true takes one long query (S > 32) per task,
+// scored in ceil(S / 32) passes per pair chained through a per-warp column
+// buffer in global memory, the last one on 16-row stripes when that is enough
+// (half the lanes' rows would be idle: 600 reads of 1100-5000 nt against 48
+// references, with the unrolled loop, 74.6 -> 53.5 ms semi-global, 75.0 ->
+// 57.3 local).  Instantiations of their own keep the register allocation of
+// the short-read path free of the long path's state.
+// Stripes are aligned so the read's last row is the last row of its last
+// stripe; the rows before the read's first row score 0 against every real
 // column and hold H = 0 exactly, the top border the first real row needs.
-template <int R, bool kLocal, bool kPanelW, bool kSmemPanel, bool kLong, bool kCheck>
-__global__ void __launch_bounds__(kK2Threads, R > 16 ? ESG_K2_R32_BLOCKS : (kPanelW ? 4 : ESG_K2_MIN_BLOCKS))
+template <int R, bool kLocal, bool kSmemPanel, bool kLong, int kLanes>
+__global__ void __launch_bounds__(kK2Threads, R > 16 ? ESG_K2_R32_BLOCKS : ESG_K2_MIN_BLOCKS)
     k2_batched(const K2Params P) {
+  constexpr bool kCheck = kLanes == kLanesChecked;
+  constexpr bool kHalf = kLanes == kLanesHalf;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ uint64_t panel_bar;
   const int lane = threadIdx.x & 31;
@@ -683,12 +730,14 @@ __global__ void __launch_bounds__(kK2Threads, R > 16 ? ESG_K2_R32_BLOCKS : (kPan
 
   const int bias = P.bias;
   PassConst K;
-  K.g0 = pack16x2(bias + P.o, bias + P.o);  // G of a zero border cell
-  K.bias2 = pack16x2(bias, bias);           // H = 0 (the local floor)
-  K.o32 = (uint32_t)(P.o * 65537);           // + o in both halves, one 32-bit add
+  // a zero border cell's G (kLanesHalf: its H) and its E and F
+  K.g0 = kHalf ? 0u : pack16x2(bias + P.o, bias + P.o);
+  K.neg2 = kHalf ? 0u : pack16x2(kNeg16, kNeg16);
+  K.bias2 = pack16x2(bias, bias);  // H = 0 (the local floor)
+  // + o in both halves: one 32-bit add, or one f16x2 add
+  K.o32 = kHalf ? half_pair(P.o) : (uint32_t)(P.o * 65537);
   K.e2 = P.e2;
   K.one = P.one;  // 1, opaque to the compiler: keeps G's add an IMAD
-  K.neg2 = pack16x2(kNeg16, kNeg16);
 
   for (;;) {
     uint32_t task = 0;
@@ -709,10 +758,15 @@ __global__ void __launch_bounds__(kK2Threads, R > 16 ? ESG_K2_R32_BLOCKS : (kPan
       const bool rc = qid >= P.n_reads;
       const uint32_t rd = rc ? qid - P.n_reads : qid;
       const uint32_t n = P.len[rd];
-      const int S = smax;
-      const int pad = S * R - (int)n;
-      const int passes = (S + 31) / 32;
-      const int owner = (S - 1) & 31;  // lane holding the last stripe
+      // passes of 32 R-row stripes; a last pass of at most 16 rows a lane
+      // takes 16-row stripes
+      const int passes = (smax + 31) / 32;
+      const int before = (passes - 1) * 32 * R;  // rows of the passes before the last
+      const bool narrow = (int)n - before <= 32 * 16;
+      const int RL = narrow ? 16 : R;
+      const int SL = ((int)n - before + RL - 1) / RL;  // stripes of the last pass
+      const int pad = before + SL * RL - (int)n;
+      const int owner = SL - 1;  // lane holding the last stripe
       const uint8_t* q = P.codes + P.off[rd];
       if (lane == owner) {
         slot[0] = INT32_MIN;
@@ -726,22 +780,27 @@ __global__ void __launch_bounds__(kK2Threads, R > 16 ? ESG_K2_R32_BLOCKS : (kPan
         const int jshort = (mB > 0 && mB < mA) ? mB - 1 : -1;
         const uint16_t* sp = sels + pm.x;
         uint32_t acc = kLocal ? K.bias2 : K.neg2, lr_last = K.neg2, amacc = K.neg2;
-        for (int pass = 0; pass < passes; ++pass) {
-          const int s = pass * 32 + lane;
-          const bool valid = s < S;
-          uint32_t ta[R];
-          uint32_t tb[kPanelW ? R : 1];
-          row_tables<R, kPanelW, false>(P, q, n, rc, valid, s, pad, ta, tb);
+        auto run = [&](auto rows, int pass, bool last) {
+          constexpr int RP = decltype(rows)::value;
+          const int s = before / RP * (last ? 1 : 0) + (last ? 0 : pass * 32) + lane;
+          const bool valid = !last || lane < SL;
+          uint32_t ta[RP];
+          const bool wild = row_records<RP>(q, n, rc, valid, s, pad, scr, ta);
           const uint32_t padmask = (s == 0) ? ((1u << pad) - 1u) : 0u;
           uint32_t v, lr, am;
-          pair_pass<R, kLocal, kPanelW, true, kSmemPanel, kCheck>(
-              P, 0u, false, ta, tb, lane, valid, s == 0, padmask, mA, jshort, sp, mA + 31, K,
-              lbuf, pass > 0, pass + 1 < passes, v, lr, am);
+          pair_pass<RP, kLocal, true, kSmemPanel, kLanes>(
+              P, scr, wild, ta, lane, valid, s == 0, padmask, mA, jshort, sp, mA + 31, K, lbuf,
+              pass > 0, !last, v, lr, am);
           acc = max16x2(acc, v);
           if constexpr (kCheck) amacc = max16x2(amacc, am);
-          if (pass + 1 == passes) lr_last = lr;
+          if (last) lr_last = lr;
           __syncwarp();  // the buffer's writes are visible to the next pass
-        }
+        };
+        for (int pass = 0; pass + 1 < passes; ++pass) run(IntConst<R>{}, pass, false);
+        if (narrow)
+          run(IntConst<16>{}, passes - 1, true);
+        else
+          run(IntConst<R>{}, passes - 1, true);
 #pragma unroll
         for (int d = 16; d; d >>= 1) acc = max16x2(acc, __shfl_xor_sync(kFull, acc, d));
         if constexpr (kCheck) {
@@ -749,7 +808,7 @@ __global__ void __launch_bounds__(kK2Threads, R > 16 ? ESG_K2_R32_BLOCKS : (kPan
           for (int d = 16; d; d >>= 1) amacc = max16x2(amacc, __shfl_xor_sync(kFull, amacc, d));
         }
         if (lane == owner)
-          fold_pair<kLocal, kCheck>(P, slot, sties, cap, pm, mB, rc, qid, acc, lr_last, amacc,
+          fold_pair<kLocal, kLanes>(P, slot, sties, cap, pm, mB, rc, qid, acc, lr_last, amacc,
                                     bias);
       }
       if (lane == owner) flush_query(P, qid, chunk, slot, sties, cap);
@@ -793,9 +852,8 @@ __global__ void __launch_bounds__(kK2Threads, R > 16 ? ESG_K2_R32_BLOCKS : (kPan
     const uint32_t rd = rc ? qid - P.n_reads : qid;
 
     uint32_t ta[R];
-    uint32_t tb[kPanelW ? R : 1];
-    const bool wild = row_tables<R, kPanelW, sc_lds<kLocal, R>()>(
-        P, valid ? P.codes + P.off[rd] : P.codes, n, rc, valid, s, pad, ta, tb, scr);
+    const bool wild =
+        row_records<R>(valid ? P.codes + P.off[rd] : P.codes, n, rc, valid, s, pad, scr, ta);
     // rows of the read's top padding (first lane only): excluded from the
     // semi-global last-column maximum
     const uint32_t padmask = (valid && first) ? ((1u << pad) - 1u) : 0u;
@@ -812,9 +870,9 @@ __global__ void __launch_bounds__(kK2Threads, R > 16 ? ESG_K2_R32_BLOCKS : (kPan
       const int mA = (int)(pm.y & 0xffffu), mB = (int)(pm.y >> 16);  // mA >= mB
       const int jshort = (mB > 0 && mB < mA) ? mB - 1 : -1;
       uint32_t v, lr, am;
-      pair_pass<R, kLocal, kPanelW, false, kSmemPanel, kCheck>(
-          P, scr, wild, ta, tb, s, valid, first, padmask, mA, jshort, sels + pm.x, mA + smax - 1,
-          K, nullptr, false, false, v, lr, am);
+      pair_pass<R, kLocal, false, kSmemPanel, kLanes>(
+          P, scr, wild, ta, s, valid, first, padmask, mA, jshort, sels + pm.x, mA + smax - 1, K,
+          nullptr, false, false, v, lr, am);
       // per-query maximum, to the query's last lane
 #pragma unroll
       for (int d = 1; d < 32; d <<= 1) {
@@ -825,7 +883,7 @@ __global__ void __launch_bounds__(kK2Threads, R > 16 ? ESG_K2_R32_BLOCKS : (kPan
           if (s >= d) am = max16x2(am, wa);
         }
       }
-      if (last) fold_pair<kLocal, kCheck>(P, slot, sties, cap, pm, mB, rc, qid, v, lr, am, bias);
+      if (last) fold_pair<kLocal, kLanes>(P, slot, sties, cap, pm, mB, rc, qid, v, lr, am, bias);
     }
 
     // --- flush the query states of this task
@@ -836,29 +894,50 @@ __global__ void __launch_bounds__(kK2Threads, R > 16 ? ESG_K2_R32_BLOCKS : (kPan
 }
 
 // ---------------------------------------------------------------- chunk merge
-// Two query states over disjoint candidate sets, each with its first
-// min(n_tied, cap) ties in candidate order, into one (mapper.rs:444-472
-// over the union): the higher best wins, equal bests add their tie counts
-// and merge their lists in candidate order.  `out` must not alias ta / tb.
-__device__ __forceinline__ int4 merge_state(int4 a, const uint32_t* ta, int4 b,
-                                            const uint32_t* tb, uint32_t cap, uint32_t* out) {
-  const uint32_t na = min((uint32_t)a.z, cap), nb = min((uint32_t)b.z, cap);
-  if (a.x > b.x) {
-    for (uint32_t k = 0; k < na; ++k) out[k] = ta[k];
-    return make_int4(a.x, max(max(a.y, b.y), b.x), a.z, a.w | b.w);
+// The 32 smallest of two sorted lists of 32 (lane k holds a list's k-th
+// smallest, kNoRef past its end), sorted: the lanewise minimum of one list
+// and the other reversed is bitonic and holds them.
+__device__ __forceinline__ uint32_t merge_lists(uint32_t a, uint32_t b, int lane) {
+  uint32_t x = min(a, __shfl_sync(kFull, b, 31 - lane));
+#pragma unroll
+  for (int d = 16; d; d >>= 1) {
+    const uint32_t y = __shfl_xor_sync(kFull, x, d);
+    x = (lane & d) ? max(x, y) : min(x, y);
   }
-  if (b.x > a.x) {
-    for (uint32_t k = 0; k < nb; ++k) out[k] = tb[k];
-    return make_int4(b.x, max(max(a.y, b.y), a.x), b.z, a.w | b.w);
+  return x;
+}
+
+// One warp: a query's panel chunks' states (heads and tie lists of the query,
+// n_chunks of them) into the state over their union (mapper.rs:444-472): the
+// highest best, its ties counted in full, the best score outside them.  Lane
+// k returns the k-th tie in candidate order.  The chunks go a lane each, so a
+// small batch cut into a chunk per reference pair pays a few loads here, not
+// a chain of them (one thread a query walked 20 chunks in about 25 us).
+__device__ __forceinline__ int4 merge_chunks(const int4* head, const uint32_t* ties,
+                                             uint32_t n_chunks, uint32_t cap, int lane,
+                                             uint32_t& tie) {
+  int best = INT32_MIN;
+  for (uint32_t c = lane; c < n_chunks; c += 32) best = max(best, head[c].x);
+  best = __reduce_max_sync(kFull, best);
+  int sub = INT32_MIN;
+  uint32_t n = 0, flags = 0;
+  tie = kNoRef;
+  for (uint32_t c0 = 0; c0 < n_chunks; c0 += 32) {
+    const uint32_t c = c0 + lane;
+    const int4 b = c < n_chunks ? head[c] : make_int4(INT32_MIN, INT32_MIN, 0, 0);
+    const bool on = c < n_chunks && b.x == best;
+    sub = max(sub, on ? b.y : b.x);
+    n += on ? (uint32_t)b.z : 0u;
+    flags |= (uint32_t)b.w;
+    for (uint32_t m = __ballot_sync(kFull, on); m; m &= m - 1) {
+      const int src = __ffs(m) - 1;
+      const uint32_t nl = min((uint32_t)__shfl_sync(kFull, b.z, src), cap);
+      const uint32_t t = (uint32_t)lane < nl ? ties[(size_t)(c0 + src) * cap + lane] : kNoRef;
+      tie = merge_lists(tie, t, lane);
+    }
   }
-  uint32_t i = 0, j = 0, w = 0;
-  while (w < cap && (i < na || j < nb)) {
-    if (j >= nb || (i < na && ta[i] < tb[j]))
-      out[w++] = ta[i++];
-    else
-      out[w++] = tb[j++];
-  }
-  return make_int4(a.x, max(a.y, b.y), a.z + b.z, a.w | b.w);
+  return make_int4(best, __reduce_max_sync(kFull, sub), (int)__reduce_add_sync(kFull, n),
+                   (int)__reduce_or_sync(kFull, flags));
 }
 
 struct KMParams {
@@ -876,27 +955,20 @@ struct KMParams {
   uint32_t redo_cap;
 };
 
-// One thread per query: its panel chunks' partial states merged in chunk
-// order, and a re-score request where any chunk may have wrapped.
+// One warp per query: its panel chunks' partial states merged, and a re-score
+// request where any chunk may have wrapped.
 static __global__ void __launch_bounds__(128) k2_merge_chunks(const KMParams P) {
-  uint32_t buf[2][kMaxCap];
-  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < P.n_order;
-       i += gridDim.x * blockDim.x) {
+  const int lane = threadIdx.x & 31;
+  const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
+  for (uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < P.n_order; i += warps) {
     const uint32_t q = P.order[i];
     const size_t base = (size_t)q * P.n_chunks;
-    const uint32_t cap = P.cap;
-    int4 acc = P.part_head[base];
-    const uint32_t n0 = min((uint32_t)acc.z, cap);
-    for (uint32_t k = 0; k < n0; ++k) buf[0][k] = P.part_ties[base * cap + k];
-    int cur = 0;
-    for (uint32_t c = 1; c < P.n_chunks; ++c) {
-      const int4 b = P.part_head[base + c];
-      acc = merge_state(acc, buf[cur], b, P.part_ties + (base + c) * cap, cap, buf[cur ^ 1]);
-      cur ^= 1;
-    }
+    uint32_t tie;
+    const int4 acc = merge_chunks(P.part_head + base, P.part_ties + base * P.cap, P.n_chunks,
+                                  P.cap, lane, tie);
+    if ((uint32_t)lane < P.cap) P.qties[(size_t)q * P.cap + lane] = tie;
+    if (lane) continue;
     P.qhead[q] = acc;
-    const uint32_t nl = min((uint32_t)acc.z, cap);
-    for (uint32_t k = 0; k < nl; ++k) P.qties[(size_t)q * cap + k] = buf[cur][k];
     if (acc.w & kQRedo) {
       const uint32_t at = atomicAdd(&P.counters[1], 1u);
       if (at < P.redo_cap)
@@ -1295,6 +1367,54 @@ static __global__ void __launch_bounds__(256) k5_merge(const K5Params P) {
     for (uint32_t k = min(n_tied, cap); k < cap; ++k) out_t[k] = kNoRef;  // ESG_NO_TIE
     if (n_tied > cap) flags |= 2;  // ESG_RESULT_TIES_TRUNCATED
     P.results[r] = make_int4(best, sub, (int)n_tied, flags);
+  }
+}
+
+// Batches in panel chunks whose queries all ran on k2 and cannot be flagged:
+// k2_merge_chunks and k5_merge in one, a warp per read.
+struct K5ChunkParams {
+  K5Params M;
+  uint32_t n_chunks;
+  const int4* part_head;
+  const uint32_t* part_ties;
+};
+
+static __global__ void __launch_bounds__(128) k5_merge_chunks(const K5ChunkParams P) {
+  const int lane = threadIdx.x & 31;
+  const uint32_t warps = (gridDim.x * blockDim.x) >> 5, cap = P.M.cap;
+  for (uint32_t r = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; r < P.M.n_reads; r += warps) {
+    uint32_t tie = kNoRef;
+    int4 out = make_int4(INT32_MIN, INT32_MIN, 0, 1 /* ESG_RESULT_EMPTY */);
+    if (P.M.len[r] == 0) {
+      if (P.M.rows)
+        for (uint32_t j = lane; j < P.M.n_refs; j += 32) {
+          P.M.rows[(size_t)r * P.M.n_refs + j] = 0;
+          if (P.M.both) P.M.rows[((size_t)P.M.n_reads + r) * P.M.n_refs + j] = 0;
+        }
+    } else {
+      size_t base = (size_t)r * P.n_chunks;
+      int4 a = merge_chunks(P.part_head + base, P.part_ties + base * cap, P.n_chunks, cap, lane,
+                            tie);
+      if (P.M.both) {
+        base += (size_t)P.M.n_reads * P.n_chunks;
+        uint32_t tb;
+        const int4 b = merge_chunks(P.part_head + base, P.part_ties + base * cap, P.n_chunks, cap,
+                                    lane, tb);
+        const int sub = max(a.y, b.y);
+        if (a.x == b.x) {
+          a = make_int4(a.x, sub, a.z + b.z, 0);
+          tie = merge_lists(tie, tb, lane);
+        } else if (a.x > b.x) {
+          a = make_int4(a.x, max(sub, b.x), a.z, 0);
+        } else {
+          a = make_int4(b.x, max(sub, a.x), b.z, 0);
+          tie = tb;
+        }
+      }
+      out = make_int4(a.x, a.y, a.z, (uint32_t)a.z > cap ? 2 : 0 /* ESG_RESULT_TIES_TRUNCATED */);
+    }
+    if ((uint32_t)lane < cap) P.M.ties[(size_t)r * cap + lane] = tie;  // kNoRef: ESG_NO_TIE
+    if (lane == 0) P.M.results[r] = out;
   }
 }
 

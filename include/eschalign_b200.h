@@ -103,7 +103,8 @@ typedef struct esg_info {
     int32_t batched_threads;  /* threads per CTA                                       */
     int32_t plain_blocks;
     int32_t plain_threads;
-    uint32_t split_len;       /* queries up to this length take 16-row stripes  */
+    uint32_t split_len;       /* queries up to this length take 16-row stripes,
+                                 longer ones (as a rule) 28- or 32-row ones     */
     int32_t tuned;            /* split_len was measured by esg_scorer_autotune   */
 } esg_info;
 
@@ -211,15 +212,19 @@ esg_status esg_scorer_autotune(esg_scorer* scorer, esg_tune_report* out);
  * reference. */
 esg_status esg_scorer_autotune_lengths(esg_scorer* scorer, const uint32_t* lens, uint32_t n,
                                        esg_tune_report* out);
-/* Set the 16/32-row split by hand (0: every query on 32-row stripes). */
+/* Set the split by hand: queries up to it take 16-row stripes, longer ones
+ * 28- or 32-row ones, whichever their length pads less (0: every query).
+ * Without this call, small batches take 8- or 16-row stripes at every length
+ * instead, for latency. */
 esg_status esg_scorer_set_split(esg_scorer* scorer, uint32_t split_len);
 
 /* Panel chunking (no counterpart in the reference): when a batch has too
  * few 32-lane tiles to keep every resident warp busy to the end (few reads,
  * or a large panel), each tile's reference pairs are cut into up to
  * `max_chunks` chunks of about equal columns, one task each, and the
- * per-chunk states are merged on the device.  1 turns it off; default 64.
- * Scores do not depend on it. */
+ * per-chunk states are merged on the device.  1 turns it off; without this
+ * call a tile has as many as the batch calls for, a reference pair each at
+ * most.  Scores do not depend on it. */
 esg_status esg_scorer_set_chunking(esg_scorer* scorer, uint32_t max_chunks);
 
 /* GpuScorer::scores_len (cuda/mod.rs:506-508): 1 for every len > 0 -- nothing

@@ -1,0 +1,67 @@
+"""The batched kernel's shapes and lane formats at their edges, against the
+scalar oracle by equality: read lengths around a stripe of 16, 28 and 32
+rows, the lengths where the shape changes (224 / 225, 1024 / 1025) and where
+a long read's last pass changes its stripes (512 rows past a pass), and
+panels whose largest score is the last the f16 lanes hold (2047) and the
+first they do not."""
+import numpy as np
+import pytest
+
+from eschalign_b200 import GpuScorer, Mode, Scoring
+from tests.test_gpu_parity import check
+
+pytestmark = pytest.mark.gpu
+
+SHORT = [1, 15, 16, 17, 27, 28, 29, 31, 32, 33, 55, 56, 57, 63, 64, 65, 111, 112, 113, 224, 225]
+LONG = [895, 897, 1023, 1024, 1025, 1535, 1536, 1537, 2047, 2048, 2049, 2560, 2561]
+DEFAULT = ((0, 16, 64), (0, 16, 1))  # KERNEL_AUTO on the default split
+
+
+def _reads(rng, panel, lens):
+    out = []
+    for k, n in enumerate(lens):
+        ref = panel[k % len(panel)]
+        r = np.resize(ref, n).copy()
+        hit = rng.random(n) < 0.08
+        r[hit] = rng.integers(0, 5 if k % 3 == 0 else 4, int(hit.sum()))
+        out.append(r.astype(np.uint8))
+    return out
+
+
+@pytest.mark.parametrize("mode", [Mode.LOCAL, Mode.SEMIGLOBAL])
+@pytest.mark.parametrize("lens,spread", [(SHORT, (1, 31, 90, 130)), (LONG, (20, 40, 300))],
+                         ids=["short", "long"])
+def test_shapes_at_their_edges(oracle, mode, lens, spread):
+    rng = np.random.default_rng(len(lens))
+    panel = [rng.integers(0, 5 if n == 90 else 4, n).astype(np.uint8) for n in spread]
+    reads = _reads(rng, panel, lens)
+    for scoring in ((2, -1, -10, -1), (3, 1, -5, -2), (2, -3, -1, -5)):
+        check(oracle, panel, reads, scoring, mode, "shape edges", kernels=DEFAULT)
+
+
+@pytest.mark.parametrize("match,length", [(23, 89), (32, 64), (89, 23), (127, 16), (127, 17)])
+def test_last_score_of_the_f16_lanes(oracle, match, length):
+    """match x length = 2047 is the largest score kept as an f16 subnormal;
+    2048 takes the int16 lanes, as does 127 x 17."""
+    rng = np.random.default_rng(match)
+    panel = [rng.integers(0, 4, length).astype(np.uint8) for _ in range(3)]
+    panel.append(np.full(length, 4, np.uint8))  # wildcards: every read scores the most
+    reads = _reads(rng, panel, [length, length - 1, length + 40, 5]) + [p.copy() for p in panel]
+    for scoring in ((match, 0, -7, -1), (match, -match + 127 - match, -1, -1)):
+        if scoring[1] < match:
+            check(oracle, panel, reads, scoring, Mode.LOCAL, "f16 limit", kernels=DEFAULT)
+
+
+def test_scorers_over_panels_of_different_sizes(oracle):
+    """A scorer over a small panel made later leaves one over a larger panel
+    (more shared memory a CTA) usable."""
+    rng = np.random.default_rng(5)
+    big = [rng.integers(0, 4, 900).astype(np.uint8) for _ in range(60)]
+    small = [rng.integers(0, 4, 50).astype(np.uint8)]
+    reads = _reads(rng, big, [40, 100, 300])
+    with GpuScorer(big, Scoring(), Mode.LOCAL) as g, GpuScorer(small, Scoring(), Mode.LOCAL) as h:
+        assert g.info()["panel_bytes"] > 48 * 1024
+        rows = g.score_batch(reads, full_rows=True).rows
+        assert (h.score_batch(reads, full_rows=True).rows ==
+                oracle.score_matrix(reads, small, (2, -1, -10, -1), True)).all()
+    assert (rows == oracle.score_matrix(reads, big, (2, -1, -10, -1), True)).all()
