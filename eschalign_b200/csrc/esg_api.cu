@@ -1651,7 +1651,9 @@ static esg_status launch_device_work(esg_scorer* sc, esg_batch* b, cudaStream_t 
     P.out = b->d_k3out;
     P.rows = rows ? b->d_rows : nullptr;
     P.wmax = plain ? 1u : 32u;
-    P.refs_per_task = 32;
+    const int k3_blocks = plain ? sc->k3_blocks1 : sc->k3_blocks;
+    P.refs_per_task = k3_refs_per_task((uint64_t)b->host_list + b->redo_cap, sc->n_refs,
+                                       (uint64_t)k3_blocks * kK3Warps);
     // counters[6..7]: the units' 64-bit counter (8-byte aligned, reset with
     // the rest each launch)
     P.task_counter = reinterpret_cast<unsigned long long*>(b->d_counters + 6);
@@ -1662,7 +1664,7 @@ static esg_status launch_device_work(esg_scorer* sc, esg_batch* b, cudaStream_t 
     P.e = sc->scoring.gap_extend;
     P.one = 1;
     void* args[] = {&P};
-    ESG_CUDA(cudaLaunchKernel(sc->k3_fn, dim3(plain ? sc->k3_blocks1 : sc->k3_blocks),
+    ESG_CUDA(cudaLaunchKernel(sc->k3_fn, dim3(k3_blocks),
                               dim3(kK3Threads), args, 0, st));
     ++kernels;
     K4Params Q{};

@@ -984,7 +984,8 @@ static __global__ void __launch_bounds__(128) k2_merge_chunks(const KMParams P) 
 // reference of the panel and writes the rows (k4 reduces them).  The work
 // unit is (query, a run of references); one warp takes one unit at a time.
 //
-// Lanes hold 16-row stripes of the query.  A query of S stripes is scored
+// Lanes hold 28- or 32-row stripes of the query, whichever k3_cost says its
+// length fills better.  A query of S stripes is scored
 // against a reference by a chain of W = min(S, wmax) lanes: the lane at
 // position w of the chain holds stripes w, W + w, 2W + w, ... in successive
 // passes, walks the reference's columns one per step, lagging the lane
@@ -998,16 +999,21 @@ static __global__ void __launch_bounds__(128) k2_merge_chunks(const KMParams P) 
 // thread per (query, reference) pair, the stripes' bottom row through the
 // buffer -- the plain comparison arm.
 //
-// Per cell: G = H + o is kept instead of H, so E, F and the diagonal term
-// are one VIADDMNMX each (max(X + e, G) and max(G_diag + (s - o), E)), H one
-// VIMNMX3 (with the zero floor in local mode), G one IMAD on the FMA pipe;
-// the substitution s - o comes from the lane's per-column record in shared
-// memory (word c = the score of read code c against this column, one
-// 16-byte table load and four stores per column), one load per cell.  The
-// query is padded at the top to whole stripes with rows that score 0, which
-// hold H = 0 exactly -- the top border -- and are left out of the
-// semi-global last-column maximum.
-constexpr int kK3Rows = 16;
+// What bounds it is the integer ALU, so a cell takes the fewest DPX
+// instructions: E, F and H one each (and half one for the local best), the
+// diagonal term G_diag + (s - o) and G = H + o as IMADs on the FMA pipe.
+// Local mode's floor comes with E (VIADDMNMX.RELU: E >= 0 changes no H), and
+// its g[r] holds the diagonal term of the row's next column.  The substitution
+// s - o comes from the lane's per-column record in shared memory (word c = the
+// score of read code c against this column, one 16-byte table load and four
+// stores per column), one load per cell.  The query is padded at the top to
+// whole stripes with rows that score 0, which hold H = 0 exactly -- the top
+// border -- and are left out of the semi-global last-column maximum.
+// Columns that every chain is inside run without the column check; unrolled
+// twice that loop measured 121 ms against 108 (both stripe heights' loops
+// share the instruction cache).  60 000 C2 reads x 164 references, both
+// strands: 143 -> 108 ms local, 150 -> 105 semi-global, one thread per pair
+// 154 -> 116, against four ALU-bound DPX instructions on 16-row stripes.
 constexpr int kK3Warps = 4;
 constexpr int kK3Threads = kK3Warps * 32;
 constexpr uint32_t kK3Stride = (uint32_t)kK3Threads * 4;  // bytes between record words
@@ -1043,23 +1049,236 @@ struct K3Params {
 
 constexpr int32_t kNoScore = INT32_MIN;
 
+// Work of a query of n rows in R-row stripes, per reference: passes over the
+// columns, at R rows and about 4 rows' worth of per-column work each, shared
+// by the warp's chains.
+__device__ __forceinline__ float k3_cost(int n, int R, int wmax) {
+  const int S = n > 0 ? (n + R - 1) / R : 1, W = min(S, wmax);
+  return (float)(((S + W - 1) / W) * (R + 4)) / (float)(32 / W);
+}
+
+// References per unit: 32 when the units then fill the resident warps twice,
+// fewer for a short list, whose time is one unit's.
+__host__ __device__ inline uint32_t k3_refs_per_task(uint64_t queries, uint32_t n_refs,
+                                                     uint64_t warps) {
+  uint32_t r = 32;
+  while (r > 4 && queries * ((n_refs + r - 1) / r) < 2 * warps) r /= 2;
+  return r;
+}
+
+// One query (n rows at qc) against references [k_lo, k_hi) of the panel.
+template <int R, bool kLocal>
+__device__ __forceinline__ void k3_unit(const K3Params& P, const int4* tab, uint32_t my, int2* buf,
+                                        uint32_t pos, uint32_t q, int n, const uint8_t* qc, bool rc,
+                                        uint32_t u, uint32_t tpq) {
+  const int lane = threadIdx.x & 31;
+  const int o = P.o, e = P.e;
+  const int S = n > 0 ? (n + R - 1) / R : 1;
+  const int W = min(S, (int)P.wmax);
+  const int C = 32 / W;                // chains in the warp
+  const int passes = (S + W - 1) / W;
+  const int c = lane / W, w = lane - c * W;
+  const int pad = S * R - n;
+  // this unit's references: its share of the query's groups of C (whole
+  // groups, so only the query's very last group can be short)
+  const uint32_t groups = (P.n_refs + (uint32_t)C - 1) / (uint32_t)C;
+  const uint32_t k_lo = (uint32_t)((uint64_t)u * groups / tpq) * (uint32_t)C;
+  const uint32_t k_hi = min((uint32_t)((uint64_t)(u + 1) * groups / tpq) * (uint32_t)C, P.n_refs);
+
+  for (uint32_t k0 = k_lo; k0 < k_hi; k0 += (uint32_t)C) {
+    const uint32_t k = k0 + (uint32_t)c;
+    const bool has = c < C && k < k_hi;
+    const uint32_t mref = has ? P.rlen[k] : 0u;
+    // (a reference longer than the column buffer's rows, or a query that
+    // needs passes without a buffer, is not scored)
+    const bool fits = mref <= P.max_cols && (passes == 1 || buf != nullptr);
+    const int m = (fits && n > 0) ? (int)mref : 0;
+    const int M = (int)__reduce_max_sync(kFull, (unsigned)m);
+    const uint8_t* rcs = has ? P.rcodes + P.roff[k] : P.rcodes;
+    // every chain's columns (chains without a reference aside): steps before
+    // this one, and past the fill, need no column check
+    const int mmin = (int)__reduce_min_sync(kFull, m > 0 ? (unsigned)m : 0xffffffffu);
+    // local: the best H over the chain's cells; semi-global: the best of
+    // the last column and (on the lane of the last stripe) the last row
+    int acc = kLocal ? 0 : kNeg32;
+    for (int pass = 0; pass < passes; ++pass) {
+      const int s = pass * W + w;
+      const bool valid = m > 0 && s < S;
+      uint32_t addr[R];
+#pragma unroll
+      for (int r = 0; r < R; ++r) {
+        const int i = s * R + r - pad;
+        uint32_t code = 5;  // padding row
+        if (valid && i >= 0) {
+          uint32_t x = rc ? qc[n - 1 - i] : qc[i];
+          x = x > 4 ? 4 : x;
+          code = (rc && x < 4) ? 3 - x : x;
+        }
+        addr[r] = my + code * kK3Stride;
+      }
+      const uint32_t padmask = (valid && s == 0) ? ((1u << pad) - 1u) : 0u;
+      const bool from_buf = valid && pass > 0 && w == 0;
+      const bool to_buf = valid && pass + 1 < passes && w == W - 1;
+      // local: d of the row's next column; semi-global: G of its last one
+      int g[R], ev[R];
+      // this column's record: the score (s - o) of read codes 0-3
+      auto record = [&](int x) {
+        const int4 tw = tab[min(x, 4)];
+        st_shared_u32(my, (uint32_t)tw.x);
+        st_shared_u32(my + kK3Stride, (uint32_t)tw.y);
+        st_shared_u32(my + 2 * kK3Stride, (uint32_t)tw.z);
+        st_shared_u32(my + 3 * kK3Stride, (uint32_t)tw.w);
+      };
+      auto score = [&](int r) { return ld_shared_u32(addr[r]); };
+      auto add = [&](int a, uint32_t b) {  // on the FMA pipe
+        return (int)mad_lo((uint32_t)a, (uint32_t)P.one, b);
+      };
+      const int last = max(m - 1, 0);
+      int x1 = valid ? rcs[0] : 0;  // the next column's code, loaded a column ahead
+      if constexpr (kLocal) {
+        record(x1);
+        x1 = valid ? rcs[min(1, last)] : 0;
+#pragma unroll
+        for (int r = 0; r < R; ++r) g[r] = add(o, score(r));
+      } else {
+#pragma unroll
+        for (int r = 0; r < R; ++r) g[r] = o;  // G of a zero border cell
+      }
+#pragma unroll
+      for (int r = 0; r < R; ++r) ev[r] = kLocal ? 0 : kNeg32;
+      int gdc = o, gbot = o, fbot = kNeg32;
+      int best = kLocal ? 0 : kNeg32;
+      int lastrow = kNeg32, lastcol = kNeg32;
+      int2 bnext = make_int2(0, 0);
+      if (from_buf) bnext = buf[c];
+      auto column = [&](auto check, int j, int gt, int ft) {
+        constexpr bool kLast = decltype(check)::value != 0;
+        if (from_buf) {
+          gt = bnext.x;
+          ft = bnext.y;
+          bnext = buf[(size_t)min(j + 1, last) * C + c];
+        }
+        record(x1);
+        x1 = rcs[min(j + (kLocal ? 2 : 1), last)];
+        int f = ft, prev = 0, h = 0;
+        if constexpr (kLocal) {
+          int up = gt;
+#pragma unroll
+          for (int r = 0; r < R; ++r) {
+            const int d = g[r];
+            h = __vimax3_s32(d, ev[r], f);
+            if (r & 1)
+              best = __vimax3_s32(best, prev, d);
+            else
+              prev = d;
+            g[r] = add(up, score(r));
+            up = add(h, (uint32_t)o);
+            ev[r] = __viaddmax_s32_relu(ev[r], e, up);  // E >= 0: the floor of H
+            f = __viaddmax_s32(f, e, up);
+          }
+          gbot = up;
+        } else {
+          int gup = gt, dn = add(gdc, score(0));
+          gdc = gt;
+#pragma unroll
+          for (int r = 0; r < R; ++r) {
+            const int d = dn;
+            if (r + 1 < R) dn = add(g[r], score(r + 1 < R ? r + 1 : r));
+            ev[r] = __viaddmax_s32(ev[r], e, g[r]);
+            f = __viaddmax_s32(f, e, gup);
+            h = __vimax3_s32(d, ev[r], f);
+            g[r] = gup = add(h, (uint32_t)o);
+          }
+          gbot = gup;
+        }
+        fbot = f;
+        if (to_buf) buf[(size_t)j * C + c] = make_int2(gbot, fbot);
+        if constexpr (!kLocal) {
+          lastrow = max(lastrow, h);
+          if (kLast && j == m - 1) {
+            int cm = kNeg32;
+#pragma unroll
+            for (int r = 0; r < R; ++r) cm = max(cm, ((padmask >> r) & 1u) ? kNeg32 : g[r]);
+            lastcol = cm - o;
+          }
+        }
+      };
+      auto top = [&](int& gt, int& ft) {
+        gt = __shfl_up_sync(kFull, gbot, 1);
+        ft = __shfl_up_sync(kFull, fbot, 1);
+        if (w == 0) {
+          gt = o;
+          ft = kNeg32;
+        }
+      };
+      const int steps = M + W - 1;
+      int t = 0;
+      // (semi-global: short of any chain's last column)
+      const int full = min(M, mmin - (kLocal ? 0 : 1));
+      if (W - 1 < full) {
+#pragma unroll 1
+        for (; t < W - 1; ++t) {
+          int gt, ft;
+          top(gt, ft);
+          const int j = t - w;
+          if (valid && (unsigned)j < (unsigned)m) column(IntConst<0>{}, j, gt, ft);
+        }
+        const int sk = valid ? w : 0;
+#pragma unroll 1
+        for (; t < full; ++t) {
+          int gt, ft;
+          top(gt, ft);
+          column(IntConst<0>{}, t - sk, gt, ft);
+        }
+      }
+#pragma unroll 1
+      for (; t < steps; ++t) {
+        int gt, ft;
+        top(gt, ft);
+        const int j = t - w;
+        if (valid && (unsigned)j < (unsigned)m) column(IntConst<1>{}, j, gt, ft);
+      }
+      __syncwarp();  // the buffer's writes are seen by the next pass
+      if (valid) {
+        if constexpr (kLocal) {
+          acc = max(acc, best);
+        } else {
+          acc = max(acc, lastcol);
+          if (s == S - 1) acc = max(acc, lastrow);
+        }
+      }
+    }
+    // the chain's maximum, to its first lane
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      const int v = __shfl_down_sync(kFull, acc, d);
+      if (w + d < W) acc = max(acc, v);
+    }
+    if (has && w == 0) {
+      // scalar.rs:123-125: an empty query or reference scores 0
+      const int score = !fits ? kNoScore : (m == 0 ? 0 : acc);
+      const uint32_t ref = P.ridx ? P.ridx[k] : k;
+      if (P.out) P.out[(size_t)pos * P.n_refs + ref] = score;
+      if (P.rows) P.rows[(size_t)q * P.n_refs + ref] = score;
+    }
+  }
+}
+
 template <bool kLocal>
-__global__ void __launch_bounds__(kK3Threads, 4) k3_lanes(const K3Params P) {
-  constexpr int R = kK3Rows;
+__global__ void __launch_bounds__(kK3Threads, 3) k3_lanes(const K3Params P) {
   __shared__ int4 tab[5];                      // words of read codes 0-3 against reference code x
   __shared__ uint32_t rec[6 * kK3Threads];     // word c of thread t at c * kK3Threads + t
   const int lane = threadIdx.x & 31;
   const int wib = threadIdx.x >> 5;
-  const int o = P.o, e = P.e;
-  const int mao = P.ma - o, mio = P.mi - o;
+  const int mao = P.ma - P.o, mio = P.mi - P.o;
   if (threadIdx.x < 5) {
     const int x = threadIdx.x;  // 4: a wildcard reference base matches every read code
     tab[x] = make_int4((x == 0 || x == 4) ? mao : mio, (x == 1 || x == 4) ? mao : mio,
                        (x == 2 || x == 4) ? mao : mio, (x == 3 || x == 4) ? mao : mio);
   }
   const uint32_t my = (uint32_t)__cvta_generic_to_shared(rec) + threadIdx.x * 4u;
-  st_shared_u32(my + 4 * kK3Stride, (uint32_t)mao);  // read wildcard: a match everywhere
-  st_shared_u32(my + 5 * kK3Stride, (uint32_t)-o);   // padding row: s = 0
+  st_shared_u32(my + 4 * kK3Stride, (uint32_t)mao);   // read wildcard: a match everywhere
+  st_shared_u32(my + 5 * kK3Stride, (uint32_t)-P.o);  // padding row: s = 0
   __syncthreads();
 
   const uint32_t n_list =
@@ -1086,142 +1305,10 @@ __global__ void __launch_bounds__(kK3Threads, 4) k3_lanes(const K3Params P) {
     const uint32_t rd = rc ? q - P.n_reads : q;
     const int n = (int)P.len[rd];
     const uint8_t* qc = P.codes + P.off[rd];
-
-    const int S = n > 0 ? (n + R - 1) / R : 1;
-    const int W = min(S, (int)P.wmax);
-    const int C = 32 / W;                // chains in the warp
-    const int passes = (S + W - 1) / W;
-    const int c = lane / W, w = lane - c * W;
-    const int pad = S * R - n;
-    // this unit's references: its share of the query's groups of C (whole
-    // groups, so only the query's very last group can be short)
-    const uint32_t groups = (P.n_refs + (uint32_t)C - 1) / (uint32_t)C;
-    const uint32_t k_lo = (uint32_t)((uint64_t)u * groups / tpq) * (uint32_t)C;
-    const uint32_t k_hi = min((uint32_t)((uint64_t)(u + 1) * groups / tpq) * (uint32_t)C, P.n_refs);
-
-    for (uint32_t k0 = k_lo; k0 < k_hi; k0 += (uint32_t)C) {
-      const uint32_t k = k0 + (uint32_t)c;
-      const bool has = c < C && k < k_hi;
-      const uint32_t mref = has ? P.rlen[k] : 0u;
-      // (a reference longer than the column buffer's rows, or a query that
-      // needs passes without a buffer, is not scored)
-      const bool fits = mref <= P.max_cols && (passes == 1 || buf != nullptr);
-      const int m = (fits && n > 0) ? (int)mref : 0;
-      const int M = (int)__reduce_max_sync(kFull, (unsigned)m);
-      const uint8_t* rcs = has ? P.rcodes + P.roff[k] : P.rcodes;
-      // local: the best H over the chain's cells; semi-global: the best of
-      // the last column and (on the lane of the last stripe) the last row
-      int acc = kLocal ? 0 : kNeg32;
-      for (int pass = 0; pass < passes; ++pass) {
-        const int s = pass * W + w;
-        const bool valid = m > 0 && s < S;
-        uint32_t addr[R];
-#pragma unroll
-        for (int r = 0; r < R; ++r) {
-          const int i = s * R + r - pad;
-          uint32_t code = 5;  // padding row
-          if (valid && i >= 0) {
-            uint32_t x = rc ? qc[n - 1 - i] : qc[i];
-            x = x > 4 ? 4 : x;
-            code = (rc && x < 4) ? 3 - x : x;
-          }
-          addr[r] = my + code * kK3Stride;
-        }
-        const uint32_t padmask = (valid && s == 0) ? ((1u << pad) - 1u) : 0u;
-        const bool from_buf = pass > 0 && w == 0;
-        const bool to_buf = pass + 1 < passes && w == W - 1;
-        int g[R], ev[R];
-#pragma unroll
-        for (int r = 0; r < R; ++r) {
-          g[r] = o;  // G of a zero border cell
-          ev[r] = kNeg32;
-        }
-        int gdc = o, gbot = o, fbot = kNeg32;
-        int best = kLocal ? 0 : kNeg32;
-        int lastrow = kNeg32, lastcol = kNeg32;
-        const int steps = M + W - 1;
-#pragma unroll 1
-        for (int t = 0; t < steps; ++t) {
-          int gt = __shfl_up_sync(kFull, gbot, 1);
-          int ft = __shfl_up_sync(kFull, fbot, 1);
-          if (w == 0) {
-            gt = o;
-            ft = kNeg32;
-          }
-          const int j = t - w;
-          if (valid && (unsigned)j < (unsigned)m) {
-            if (from_buf) {
-              const int2 b = buf[(size_t)j * C + c];
-              gt = b.x;
-              ft = b.y;
-            }
-            // this column's record: the score (s - o) of read codes 0-3
-            const int x = min((int)rcs[j], 4);
-            const int4 tw = tab[x];
-            st_shared_u32(my, (uint32_t)tw.x);
-            st_shared_u32(my + kK3Stride, (uint32_t)tw.y);
-            st_shared_u32(my + 2 * kK3Stride, (uint32_t)tw.z);
-            st_shared_u32(my + 3 * kK3Stride, (uint32_t)tw.w);
-            int gd = gdc;
-            gdc = gt;
-            int gup = gt, f = ft, hprev = 0, hlast = 0;
-#pragma unroll
-            for (int r = 0; r < R; ++r) {
-              const int sc = (int)ld_shared_u32(addr[r]);
-              ev[r] = __viaddmax_s32(ev[r], e, g[r]);
-              f = __viaddmax_s32(f, e, gup);
-              const int h1 = __viaddmax_s32(gd, sc, ev[r]);
-              int h;
-              if constexpr (kLocal) {
-                h = __vimax3_s32(h1, f, 0);
-                if (r & 1)
-                  best = __vimax3_s32(best, hprev, h);
-                else
-                  hprev = h;
-              } else {
-                h = max(h1, f);
-              }
-              gd = g[r];
-              g[r] = (int)mad_lo((uint32_t)h, (uint32_t)P.one, (uint32_t)o);
-              gup = g[r];
-              if (r == R - 1) hlast = h;
-            }
-            gbot = g[R - 1];
-            fbot = f;
-            if (to_buf) buf[(size_t)j * C + c] = make_int2(gbot, fbot);
-            if constexpr (!kLocal) {
-              lastrow = max(lastrow, hlast);
-              if (j == m - 1) {
-                int cm = kNeg32;
-#pragma unroll
-                for (int r = 0; r < R; ++r) cm = max(cm, ((padmask >> r) & 1u) ? kNeg32 : g[r]);
-                lastcol = cm - o;
-              }
-            }
-          }
-        }
-        __syncwarp();  // the buffer's writes are seen by the next pass
-        if constexpr (kLocal) {
-          acc = max(acc, best);
-        } else {
-          acc = max(acc, lastcol);
-          if (valid && s == S - 1) acc = max(acc, lastrow);
-        }
-      }
-      // the chain's maximum, to its first lane
-#pragma unroll
-      for (int d = 1; d < 32; d <<= 1) {
-        const int v = __shfl_down_sync(kFull, acc, d);
-        if (w + d < W) acc = max(acc, v);
-      }
-      if (has && w == 0) {
-        // scalar.rs:123-125: an empty query or reference scores 0
-        const int score = !fits ? kNoScore : (m == 0 ? 0 : acc);
-        const uint32_t ref = P.ridx ? P.ridx[k] : k;
-        if (P.out) P.out[(size_t)pos * P.n_refs + ref] = score;
-        if (P.rows) P.rows[(size_t)q * P.n_refs + ref] = score;
-      }
-    }
+    if (k3_cost(n, 28, (int)P.wmax) < k3_cost(n, 32, (int)P.wmax))
+      k3_unit<28, kLocal>(P, tab, my, buf, pos, q, n, qc, rc, u, tpq);
+    else
+      k3_unit<32, kLocal>(P, tab, my, buf, pos, q, n, qc, rc, u, tpq);
   }
 }
 

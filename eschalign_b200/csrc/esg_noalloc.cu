@@ -103,7 +103,7 @@ extern "C" esg_status esg_score_rows_noalloc(const uint8_t* d_codes, const uint6
   // one reference's bottom row (max_ref_len columns) per warp must fit the
   // static array: at most kScratchInt2 / max_ref_len warps
   const size_t cols = max_ref_len ? max_ref_len : 1;
-  size_t blocks = std::min<size_t>((size_t)sms * 4, kScratchInt2 / (cols * kK3Warps));
+  size_t blocks = std::min<size_t>((size_t)sms * 3, kScratchInt2 / (cols * kK3Warps));
   if (blocks == 0) blocks = 1;  // max_ref_len <= 8192 keeps 64 CTAs in bounds
   K3Params P{};
   P.codes = d_codes;
@@ -121,7 +121,7 @@ extern "C" esg_status esg_score_rows_noalloc(const uint8_t* d_codes, const uint6
   P.out = nullptr;
   P.rows = d_rows;
   P.wmax = 32;
-  P.refs_per_task = 32;
+  P.refs_per_task = k3_refs_per_task(n_queries, n_refs, (uint64_t)blocks * kK3Warps);
   P.task_counter = nullptr;  // units taken warp-strided: no counter to clear
   P.colbuf = scratch;
   P.ma = s.match_score;

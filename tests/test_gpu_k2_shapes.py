@@ -14,6 +14,7 @@ pytestmark = pytest.mark.gpu
 
 SHORT = [1, 15, 16, 17, 27, 28, 29, 31, 32, 33, 55, 56, 57, 63, 64, 65, 111, 112, 113, 224, 225]
 LONG = [895, 897, 1023, 1024, 1025, 1535, 1536, 1537, 2047, 2048, 2049, 2560, 2561]
+INT32 = ((2, 256, 64), (1, 256, 64))  # KERNEL_INT32, KERNEL_PLAIN32
 DEFAULT = ((0, 16, 64), (0, 16, 1))  # KERNEL_AUTO on the default split
 
 
@@ -37,6 +38,19 @@ def test_shapes_at_their_edges(oracle, mode, lens, spread):
     reads = _reads(rng, panel, lens)
     for scoring in ((2, -1, -10, -1), (3, 1, -5, -2), (2, -3, -1, -5)):
         check(oracle, panel, reads, scoring, mode, "shape edges", kernels=DEFAULT)
+
+
+@pytest.mark.parametrize("mode", [Mode.LOCAL, Mode.SEMIGLOBAL])
+def test_int32_lanes_at_their_edges(oracle, mode):
+    """Chains of 1-32 lanes, one to four passes, one reference and lists
+    short enough for fewer references a unit."""
+    rng = np.random.default_rng(32)
+    panel = [rng.integers(0, 5 if n == 40 else 4, n).astype(np.uint8) for n in (1, 2, 31, 40, 300)]
+    reads = _reads(rng, panel, SHORT + [896, 897, 1024, 1025, 3073])
+    for scoring in ((100, -100, -200, -30), (2, -3, -1, -5)):
+        check(oracle, panel, reads, scoring, mode, "int32 edges", kernels=INT32)
+        check(oracle, panel[3:4], reads[8:11], scoring, mode, "int32, one reference",
+              kernels=INT32)
 
 
 @pytest.mark.parametrize("match,length", [(23, 89), (32, 64), (89, 23), (127, 16), (127, 17)])
