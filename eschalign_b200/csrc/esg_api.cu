@@ -125,6 +125,27 @@ struct PinnedPool {
   }
 };
 
+// Per device: how many scorers there are, and the pool their tracebacks take
+// their scratch from (stream-ordered, so calls on several streams or threads
+// each get memory no other uses).
+constexpr int kMaxDevices = 64;
+std::mutex g_trace_mu;
+struct TracePool {
+  int scorers = 0;
+  cudaMemPool_t pool = nullptr;
+} g_trace[kMaxDevices];
+
+void trace_pool_ref(int device, int by) {
+  if (device < 0 || device >= kMaxDevices) return;
+  std::lock_guard<std::mutex> lk(g_trace_mu);
+  TracePool& t = g_trace[device];
+  t.scorers += by;
+  if (t.scorers == 0 && t.pool) {
+    cudaMemPoolDestroy(t.pool);
+    t.pool = nullptr;
+  }
+}
+
 struct Pinned {
   void* p = nullptr;
   size_t cap = 0;
@@ -579,6 +600,7 @@ esg_status esg_scorer_new(int32_t device, const uint8_t* ref_codes, const uint64
 
   auto* sc = new esg_scorer();
   sc->device = device;
+  trace_pool_ref(device, 1);
   sc->scoring = s;
   sc->mode = mode;
   sc->kernel = kernel;
@@ -588,11 +610,13 @@ esg_status esg_scorer_new(int32_t device, const uint8_t* ref_codes, const uint64
   sc->panel_bases = bases;
   cudaDeviceProp prop{};
   if (cudaGetDeviceProperties(&prop, device) != cudaSuccess) {
+    trace_pool_ref(device, -1);
     delete sc;
     return cuda_fail(cudaGetLastError(), "cudaGetDeviceProperties");
   }
   sc->sm_count = prop.multiProcessorCount;
   if (prop.major < 10) {
+    trace_pool_ref(device, -1);
     delete sc;
     return fail(ESG_ERR_UNAVAILABLE,
                 "device %d (%s, sm_%d%d) is not a Blackwell sm_100 part this library is built for",
@@ -602,6 +626,7 @@ esg_status esg_scorer_new(int32_t device, const uint8_t* ref_codes, const uint64
     sc->stream = (cudaStream_t)ext_stream;
   } else {
     if (cudaStreamCreateWithFlags(&sc->stream, cudaStreamNonBlocking) != cudaSuccess) {
+      trace_pool_ref(device, -1);
       delete sc;
       return cuda_fail(cudaGetLastError(), "cudaStreamCreate");
     }
@@ -840,6 +865,7 @@ void esg_scorer_free(esg_scorer* sc) {
   for (auto& ge : sc->graph_execs) cudaGraphExecDestroy(ge.second);
   if (sc->pool) cudaMemPoolDestroy(sc->pool);
   if (sc->own_stream && sc->stream) cudaStreamDestroy(sc->stream);
+  trace_pool_ref(sc->device, -1);
   delete sc;
 }
 
@@ -1442,6 +1468,25 @@ size_t esg_internal_pool_spare(esg_scorer* sc) {
       cudaMemPoolGetAttribute(sc->pool, cudaMemPoolAttrUsedMemCurrent, &used) != cudaSuccess)
     return 0;
   return reserved > used ? (size_t)(reserved - used) : 0;
+}
+
+cudaMemPool_t esg_internal_trace_pool(int device, uint64_t keep, cudaMemPool_t other) {
+  if (device < 0 || device >= kMaxDevices) return other;
+  std::lock_guard<std::mutex> lk(g_trace_mu);
+  TracePool& t = g_trace[device];
+  if (!t.pool) {
+    cudaMemPoolProps props{};
+    props.allocType = cudaMemAllocationTypePinned;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id = device;
+    if (cudaMemPoolCreate(&t.pool, &props) != cudaSuccess) {
+      cudaGetLastError();
+      t.pool = nullptr;
+      return other;
+    }
+    cudaMemPoolSetAttribute(t.pool, cudaMemPoolAttrReleaseThreshold, &keep);
+  }
+  return t.pool;
 }
 
 int esg_internal_device(const esg_scorer* sc) { return sc ? sc->device : 0; }

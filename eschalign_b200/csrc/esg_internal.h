@@ -33,6 +33,11 @@ struct esg_internal_panel {
 };
 ESG_HIDDEN void esg_internal_panel_of(esg_scorer* sc, esg_internal_panel* out);
 
+// The memory pool for the traceback's scratch on `device`: one for all its
+// scorers, keeping up to `keep` bytes between calls, gone with the last of
+// them.  `other` if it cannot be made.
+ESG_HIDDEN cudaMemPool_t esg_internal_trace_pool(int device, uint64_t keep, cudaMemPool_t other);
+
 // A submitted batch's reads on the device (NULL codes if not submitted).
 ESG_HIDDEN void esg_internal_batch_reads(const esg_batch* b, const uint8_t** codes,
                                          const uint64_t** off, const uint32_t** len,

@@ -2,6 +2,8 @@
 // (coordinates and CIGAR) of chosen (read, reference, strand) jobs, as
 // crates/eschalign/src/scalar.rs:182-364 computes it.
 //
+// k7_tags: tiles of jobs of at most 1024 rows whose scores fit 16 bits; the
+// trace rides in the low bits of the recurrence's values (see below).
 // k7_trace: one warp per task.  A task is a tile of jobs whose 16-row
 // stripes fill the warp's lanes (a job of n rows takes ceil(n / 16) lanes;
 // each job has its own reference), or one long job (over 32 stripes) run in
@@ -322,6 +324,357 @@ __global__ void __launch_bounds__(kTThreads) k7_trace(const K7Params P) {
   }
 }
 
+// ---------------------------------------------------------------- k7_tags
+// The traceback of jobs of at most 1024 rows whose scores fit 16 bits (what
+// is left takes k7_trace): tiles of jobs on 28- or 32-row stripes, one pass.
+//
+// k7_trace compares its way to a trace code, some 25 ALU instructions a cell.
+// Here the maxima of the recurrence carry it: every value is
+//     (score - 1) << 16 | source << 14 | length
+// with source 1 deletion, 2 insertion, 3 diagonal -- the order that breaks
+// ties as scalar.rs:259-285 does -- and length the gap's extensions so far.
+// Extending adds (e << 16) + 1, so on a tie the extension wins, and a gap's
+// end holds its whole length: the 16 low bits of H are all the walk needs of a
+// cell, two cells to a stored word.  A local score of 0 is the floor value 0
+// (VIADDMNMX.RELU on E), source 0: stop.  The score alone, for the next
+// cells, is (value + 0xc000) & 0xffff0000; semi-global, where no value is 0,
+// it is the high half itself (score - 1).  5 ALU instructions a cell local, 4
+// semi-global, the adds on the FMA pipe.
+// Stored words are indexed by step, not by column, so that a warp's stores
+// are contiguous: word q of lane l at step t at ((t * 4 + q) * 32 + l) * 16
+// bytes, rows 8 q .. 8 q + 7 of the stripe.
+// What bounds it: issue slots (11 instructions a cell) and the walk's loads;
+// the scratch (2 bytes a cell) is written once, 3.5 GB of DRAM traffic here.
+// 100 000 jobs of ~110 nt x 70-180 nt: 2.9 -> 1.2 ms semi-global, 3.7 -> 1.2
+// local.
+constexpr int kTagRows = 1024;    // longest read
+constexpr int kTagCols = 1700;    // longest reference: 592 warps' scratch in kTagBytes
+constexpr uint64_t kTagBytes = 2ull << 30;
+constexpr int kTagScore = 30000;  // bound on |score|, gap floors included
+constexpr int kAhead = 8;         // cells of the walk read at once (4, 8, 16: 1.24, 1.19, 1.27 ms)
+constexpr int kTagNeg = -31000 * 65536;
+constexpr uint32_t kTag28 = 0x8000u;  // in a task's count: 28-row stripes
+
+template <bool kOn>
+struct TagCheck {
+  static constexpr bool value = kOn;
+};
+
+struct K7TagParams {
+  K7Params J;
+  uint4* trace;     // per warp: steps * 128 uint4
+  uint32_t steps;   // of a tile at most
+  int one;          // 1, opaque to the compiler (keeps adds on the FMA pipe)
+};
+
+__device__ __forceinline__ uint32_t tag_lds(uint32_t a) {
+  uint32_t v;
+  asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(a));
+  return v;
+}
+__device__ __forceinline__ void tag_sts(uint32_t a, uint32_t v) {
+  asm volatile("st.shared.u32 [%0], %1;" ::"r"(a), "r"(v));
+}
+
+template <int R, bool kLocal>
+__device__ __forceinline__ void tag_tile(const K7TagParams& P, const int4* tab, uint32_t my,
+                                         uint4* trace, uint2 tk) {
+  constexpr uint32_t kStride = kTThreads * 4;
+  const K7Params& J = P.J;
+  const int lane = threadIdx.x & 31;
+  const uint32_t count = tk.y & 0x7fffu;
+  const int smax = (int)(tk.y >> 16);
+  // --- lane -> (job, stripe)
+  uint32_t job = 0, n = 0;
+  int S = 0, s0 = 0;
+  bool valid = false;
+  {
+    uint32_t kj = 0, kn = 0, kS = 0;
+    if ((uint32_t)lane < count) {
+      kj = J.order[tk.x + lane];
+      kn = J.len[J.job_q[kj] & 0x7fffffffu];
+      kS = (kn + R - 1) / R;
+    }
+    uint32_t incl = kS;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      const uint32_t v = __shfl_up_sync(kFullT, incl, d);
+      if (lane >= d) incl += v;
+    }
+    for (uint32_t k = 0; k < count; ++k) {
+      const uint32_t ek = __shfl_sync(kFullT, incl, k);
+      const uint32_t sk = __shfl_sync(kFullT, kS, k);
+      const uint32_t jk = __shfl_sync(kFullT, kj, k);
+      const uint32_t nk = __shfl_sync(kFullT, kn, k);
+      if ((uint32_t)lane >= ek - sk && (uint32_t)lane < ek) {
+        job = jk;
+        n = nk;
+        S = (int)sk;
+        s0 = (int)(ek - sk);
+        valid = true;
+      }
+    }
+  }
+  const uint32_t jq = valid ? J.job_q[job] : 0u;
+  const uint32_t rd = jq & 0x7fffffffu;
+  const bool rc = (jq >> 31) != 0;
+  const uint32_t slot = valid ? J.job_slot[job] : 0u;
+  const int m = valid ? (int)J.rlen[slot] : 0;
+  const uint8_t* rp = J.rcodes + (valid ? J.roff[slot] : 0u);
+  const uint8_t* q = J.codes + (valid ? J.off[rd] : 0ull);
+  const int pad = S * R - (int)n;
+  const int s = valid ? lane - s0 : 0;
+  const bool first = !valid || s == 0;
+  const int padrows = (valid && s == 0) ? pad : 0;
+  uint32_t addr[R];
+#pragma unroll
+  for (int r = 0; r < R; ++r) {
+    const int i = s * R + r - pad;
+    uint32_t c = 5;  // padding row
+    if (valid && i >= 0) {
+      uint32_t x = rc ? q[n - 1 - i] : q[i];
+      x = x > 4 ? 4 : x;
+      c = (rc && x < 4) ? 3 - x : x;
+    }
+    addr[r] = my + c * kStride;
+  }
+  auto add = [&](int a, int b) {  // on the FMA pipe
+    int d;
+    asm("mad.lo.s32 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(P.one), "r"(b));
+    return d;
+  };
+  const int last = max(m - 1, 0);
+  // a zero cell's score as the next cells take it
+  constexpr int kZero = kLocal ? 0 : -65536;
+  const int cE = J.o * 65536 + (kLocal ? -0xc000 : 0x4000);
+  const int cF = J.o * 65536 + (kLocal ? -0x8000 : 0x8000);
+  const int ext = J.e * 65536 + 1;
+  auto record = [&](int x) {
+    const int4 tw = tab[min(x, 4)];
+    tag_sts(my, (uint32_t)tw.x);
+    tag_sts(my + kStride, (uint32_t)tw.y);
+    tag_sts(my + 2 * kStride, (uint32_t)tw.z);
+    tag_sts(my + 3 * kStride, (uint32_t)tw.w);
+  };
+  // d of the row's next column
+  int g[R], ev[R];
+  record(valid ? rp[0] : 0);
+#pragma unroll
+  for (int r = 0; r < R; ++r) {
+    g[r] = add(kZero, (int)tag_lds(addr[r]));
+    ev[r] = kLocal ? 0 : kTagNeg;
+  }
+  int x1 = rp[min(1, last)];
+  int hbot = kZero, fbot = add(kZero, cF);
+  const int ftop = fbot;  // F of a first row: opened at the border
+  int best = kLocal ? 0 : kNegT, bj = 0, bi = 0;  // 1-based end cell, 0: none
+  const int steps = [&] {
+    int v = valid ? m + s : 0;
+    return __reduce_max_sync(kFullT, v);
+  }();
+  // columns every job's lanes are inside, short of any last column
+  const int full = (int)__reduce_min_sync(kFullT, valid ? (unsigned)(m - 1) : 0x7fffffffu);
+  auto column = [&](auto check, int t, int j, int up, int f) {
+    constexpr bool kCheck = decltype(check)::value;
+    record(x1);
+    x1 = rp[min(j + 2, last)];
+    int hc[R];
+    uint32_t w[R / 2];
+    int prev = 0, xp = 0, cm = kTagNeg;
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      const int x = __vimax3_s32(g[r], ev[r], f);
+      const int h = (kLocal ? add(x, 0xc000) : x) & (int)0xffff0000;
+      g[r] = add(up, (int)tag_lds(addr[r]));
+      ev[r] = kLocal ? __viaddmax_s32_relu(ev[r], ext, add(h, cE))
+                     : __viaddmax_s32(ev[r], ext, add(h, cE));
+      f = __viaddmax_s32(f, ext, add(h, cF));
+      up = h;
+      // the column's best, the smallest row first
+      if constexpr (kLocal) {
+        const int y = add(h, R - 1 - r);
+        if (r & 1)
+          cm = __vimax3_s32(cm, prev, y);
+        else
+          prev = y;
+      }
+      if (kCheck && !kLocal) hc[r] = h;
+      if (r & 1)
+        w[r / 2] = __byte_perm((uint32_t)xp, (uint32_t)x, 0x5410);
+      else
+        xp = x;
+    }
+    hbot = up;
+    fbot = f;
+    uint4* at = trace + (size_t)t * 128 + lane;
+#pragma unroll
+    for (int k = 0; k < R / 8; ++k)
+      at[k * 32] = make_uint4(w[4 * k], w[4 * k + 1], w[4 * k + 2], w[4 * k + 3]);
+    if constexpr (R % 8 != 0)
+      *reinterpret_cast<uint2*>(at + R / 8 * 32) = make_uint2(w[R / 8 * 4], w[R / 8 * 4 + 1]);
+    if constexpr (kLocal) {
+      if ((cm >> 16) > best) {  // padding rows hold 0: never above best
+        best = cm >> 16;
+        bi = s * R + (R - 1 - (cm & 0xffff)) - pad + 1;
+        bj = j + 1;
+      }
+    } else {
+      if (!kCheck || j < m - 1) {
+        if (s == S - 1 && (up >> 16) + 1 > best) {  // the last row
+          best = (up >> 16) + 1;
+          bi = (int)n;
+          bj = j + 1;
+        }
+      } else if constexpr (kCheck) {
+#pragma unroll
+        for (int r = 0; r < R; ++r)  // the last column, rows in order
+          if (r >= padrows && (hc[r] >> 16) + 1 > best) {
+            best = (hc[r] >> 16) + 1;
+            bi = s * R + r - pad + 1;
+            bj = m;
+          }
+      }
+    }
+  };
+  auto top = [&](int& ht, int& ft) {
+    ht = __shfl_up_sync(kFullT, hbot, 1);
+    ft = __shfl_up_sync(kFullT, fbot, 1);
+    if (first) {
+      ht = kZero;
+      ft = ftop;
+    }
+  };
+  int t = 0;
+  const int fill = smax - 1;
+  if (fill < full) {
+#pragma unroll 1
+    for (; t < fill; ++t) {
+      int ht, ft;
+      top(ht, ft);
+      const int j = t - s;
+      if (valid && (unsigned)j < (unsigned)m) column(TagCheck<true>{}, t, j, ht, ft);
+    }
+#pragma unroll 1
+    for (; t < full; ++t) {
+      int ht, ft;
+      top(ht, ft);
+      column(TagCheck<false>{}, t, t - s, ht, ft);
+    }
+  }
+#pragma unroll 1
+  for (; t < steps; ++t) {
+    int ht, ft;
+    top(ht, ft);
+    const int j = t - s;
+    if (valid && (unsigned)j < (unsigned)m) column(TagCheck<true>{}, t, j, ht, ft);
+  }
+  __syncwarp();  // trace writes visible to the warp
+  // --- the job's end cell: first maximum over its lanes
+#pragma unroll
+  for (int d = 1; d < 32; d <<= 1) {
+    const int b2 = __shfl_up_sync(kFullT, best, d);
+    const int j2 = __shfl_up_sync(kFullT, bj, d);
+    const int i2 = __shfl_up_sync(kFullT, bi, d);
+    if (valid && s >= d && better(b2, j2, i2, best, bj, bi)) {
+      best = b2;
+      bj = j2;
+      bi = i2;
+    }
+  }
+  // --- the walk, by the job's last lane.  Up to kAhead cells down the
+  // diagonal at a time -- most steps are diagonal, and their loads then wait together
+  // -- and one gap.  The walkers of a tile stay together: a branch a step for
+  // each of them took as long as the columns (34 000 instructions a tile).
+  const bool walker = valid && s == S - 1;
+  int i = walker ? bi : 0, j = walker ? bj : 0;
+  uint32_t* out = J.ops + (walker ? J.job_at[job] : 0ull);
+  uint32_t runs = 0, cur = 4, cnt = 0;
+  auto emit = [&](uint32_t op, uint32_t len) {
+    const bool flush = len && op != cur;
+    if (flush && cnt) out[runs] = (cnt << 4) | cur;
+    runs += flush && cnt;
+    cnt = (flush ? 0u : cnt) + len;
+    cur = flush ? op : cur;
+  };
+  auto code = [&](int k) -> uint32_t {  // k cells down the diagonal; 0 past the border
+    const int ip = i - k - 1 + pad, st = ip / R, r = ip - st * R;
+    const uint4* cell = trace + (size_t)(j - k - 1 + st) * 128 + (r >> 3) * 32 + (s0 + st);
+    return i > k && j > k ? (uint32_t)reinterpret_cast<const uint16_t*>(cell)[r & 7] : 0u;
+  };
+  while (__any_sync(kFullT, i > 0 && j > 0)) {
+    uint32_t cell[kAhead];
+#pragma unroll
+    for (int k = 0; k < kAhead; ++k) cell[k] = code(k);
+    int nm = 0;
+    uint32_t c = 0xc000u;  // the first that is not diagonal
+#pragma unroll
+    for (int k = 0; k < kAhead; ++k) {
+      c = c >= 0xc000u ? cell[k] : c;
+      nm += c >= 0xc000u;
+    }
+    emit(kOpM, (uint32_t)nm);
+    i -= nm;
+    j -= nm;
+    const bool on = i > 0 && j > 0, ins = c >= 0x8000u, stop = on && c < 0x4000u;
+    // (a gap from the border may count padding rows above the read)
+    const int len = on && !stop && nm < kAhead ? min((int)(c & 0x3fffu) + 1, ins ? i : j) : 0;
+    emit(ins ? kOpI : kOpD, (uint32_t)len);
+    i -= ins ? len : 0;
+    j -= ins ? 0 : len;
+    if (__any_sync(kFullT, stop)) {
+      if (stop) {  // the alignment starts here
+        const bool none = bi == 0 || bj == 0;
+        J.res[job] = none ? make_int4(0, 0, 0, 0) : make_int4(best, i, bi, j);
+        i = -1;
+      }
+    }
+  }
+  if (walker) {
+    if (cnt) out[runs++] = (cnt << 4) | cur;
+    for (uint32_t a = 0, b = runs ? runs - 1 : 0; a < b; ++a, --b) {  // first to last
+      const uint32_t x = out[a];
+      out[a] = out[b];
+      out[b] = x;
+    }
+    const bool none = bi == 0 || bj == 0;
+    if (i >= 0) J.res[job] = none ? make_int4(0, 0, 0, 0) : make_int4(best, i, bi, j);
+    J.res2[job] = make_int4(none ? 0 : bj, (int)runs, 0, 0);
+  }
+  __syncwarp();  // the walk is done before the scratch is reused
+}
+
+template <bool kLocal>
+__global__ void __launch_bounds__(kTThreads, 3) k7_tags(const K7TagParams P) {
+  __shared__ int4 tab[5];                   // words of read codes 0-3 against reference code x
+  __shared__ uint32_t rec[6 * kTThreads];   // word c of thread t at c * kTThreads + t
+  const int lane = threadIdx.x & 31;
+  // a diagonal step's addend: the score and the source
+  const int dg = kLocal ? -0x4000 : 0xc000;
+  const int ma = P.J.ma * 65536 + dg, mi = P.J.mi * 65536 + dg;
+  if (threadIdx.x < 5) {
+    const int x = threadIdx.x;  // 4: a wildcard reference base matches every read code
+    tab[x] = make_int4((x == 0 || x == 4) ? ma : mi, (x == 1 || x == 4) ? ma : mi,
+                       (x == 2 || x == 4) ? ma : mi, (x == 3 || x == 4) ? ma : mi);
+  }
+  const uint32_t my = (uint32_t)__cvta_generic_to_shared(rec) + threadIdx.x * 4u;
+  tag_sts(my + 4 * kTThreads * 4, (uint32_t)ma);  // read wildcard: a match everywhere
+  tag_sts(my + 5 * kTThreads * 4, (uint32_t)dg);  // padding row: s = 0
+  __syncthreads();
+  uint4* trace = P.trace + ((size_t)blockIdx.x * kTWarps + (threadIdx.x >> 5)) *
+                               (size_t)P.steps * 128;
+  for (;;) {
+    uint32_t task = 0;
+    if (lane == 0) task = atomicAdd(P.J.task_counter, 1u);
+    task = __shfl_sync(kFullT, task, 0);
+    if (task >= P.J.n_tasks) break;
+    const uint2 tk = P.J.tasks[task];
+    if (tk.y & kTag28)
+      tag_tile<28, kLocal>(P, tab, my, trace, tk);
+    else
+      tag_tile<32, kLocal>(P, tab, my, trace, tk);
+  }
+}
+
 // Pack each job's CIGAR words from the staging into the caller's layout.
 __global__ void __launch_bounds__(256) k7_compact(const uint32_t* staging, const uint64_t* at,
                                                   const uint64_t* dst, const int4* res2,
@@ -364,11 +717,16 @@ esg_status align_impl(esg_scorer* sc, const uint8_t* d_codes, const uint64_t* d_
   esg_internal_panel_of(sc, &P);
   if (n_jobs && (!jobs || !out)) return terr(ESG_ERR_BAD_ARGUMENT, "jobs/out must not be NULL");
   // --- plan on the host
-  std::vector<uint32_t> job_q(n_jobs), job_slot(n_jobs), S(n_jobs), M(n_jobs);
+  std::vector<uint32_t> job_q(n_jobs), job_slot(n_jobs), S(n_jobs);
   std::vector<uint64_t> job_at(n_jobs);
   uint64_t staging = 0;
-  uint32_t mcols = 1, passes_max = 1;
-  std::vector<uint32_t> live;
+  uint32_t mcols = 1, passes_max = 1, tag_cols = 1, tag_stripes = 1;
+  uint32_t all_cols = 1, all_passes = 1;  // over every job, as k7_trace would hold them
+  // jobs by kernel and stripe height: k7_tags on 28 and 32 rows, k7_trace
+  enum { kT28, kT32, kFull, kKinds };
+  std::vector<uint32_t> live[kKinds];
+  const int64_t mm = std::max(std::abs(P.scoring.match_score), std::abs(P.scoring.mismatch)),
+                go = std::abs(P.scoring.gap_open), ge = std::abs(P.scoring.gap_extend);
   for (uint32_t k = 0; k < n_jobs; ++k) {
     const esg_align_job& jb = jobs[k];
     if (jb.read >= n_reads) return terr(ESG_ERR_BAD_ARGUMENT, "job %u: no read %u", k, jb.read);
@@ -380,77 +738,110 @@ esg_status align_impl(esg_scorer* sc, const uint8_t* d_codes, const uint64_t* d_
     job_at[k] = staging;
     staging += (uint64_t)n + m + 1;
     S[k] = (n + kTR - 1) / kTR;
-    M[k] = m;
-    if (n && m) {
-      live.push_back(k);
+    if (S[k] > 0xffffu) return terr(ESG_ERR_BAD_ARGUMENT, "job %u: read too long", k);
+    if (!n || !m) continue;
+    all_cols = std::max(all_cols, m);
+    all_passes = std::max(all_passes, (S[k] + 31) / 32);
+    if (n <= kTagRows && m <= kTagCols &&
+        (int64_t)std::min(n, m) * (mm + ge) + 2 * go + mm <= kTagScore) {
+      // 28-row stripes where they pad enough less (a row costs 1.045 of a
+      // 32-row stripe's in the scoring kernel, whose loop this is)
+      const bool r28 = n <= 28 * 8 && (n + 27) / 28 * 28 * 1045 < (n + 31) / 32 * 32 * 1000;
+      S[k] = r28 ? (n + 27) / 28 : (n + 31) / 32;
+      live[r28 ? kT28 : kT32].push_back(k);
+      tag_stripes = std::max(tag_stripes, S[k]);
+      tag_cols = std::max(tag_cols, m);
+    } else {
+      live[kFull].push_back(k);
       mcols = std::max(mcols, m);
       if (S[k] > 32) passes_max = std::max(passes_max, (S[k] + 31) / 32);
     }
-    if (S[k] > 0xffffu) return terr(ESG_ERR_BAD_ARGUMENT, "job %u: read too long", k);
   }
-  // tiles of jobs up to 32 stripes (next fit, longest first); longer jobs alone
-  {
+  // tiles of jobs up to 32 stripes (next fit, longest first); longer jobs
+  // alone.  Tasks of a kernel lie together: k7_tags' first.
+  std::vector<uint32_t> order;
+  std::vector<uint2> tasks;
+  order.reserve(n_jobs);
+  uint32_t n_tag = 0;
+  for (int kind = 0; kind < kKinds; ++kind) {
+    if (kind == kFull) n_tag = (uint32_t)tasks.size();
+    std::vector<uint32_t>& lv = live[kind];
+    if (lv.empty()) continue;
     // longest first, stable: a counting sort on the stripes (long jobs, over
-    // 32 stripes, are few and sorted apart)
-    std::vector<uint32_t> longs, cnt(34, 0), sorted(live.size());
-    for (uint32_t k : live) ++cnt[std::min<uint32_t>(S[k], 33)];
+    // 32 stripes, are few and sorted apart).  k7_tags' jobs by reference
+    // length before that: a tile runs for its longest reference, and with
+    // references of 70-180 nt in any order 30 % of its lanes' steps were idle
+    std::vector<uint32_t> cnt(34, 0), start(34, 0), sorted(lv.size());
+    if (kind != kFull) {
+      std::vector<uint32_t> first(tag_cols + 2, 0);
+      auto len = [&](uint32_t k) { return P.len_of[jobs[k].ref]; };
+      for (uint32_t k : lv) ++first[tag_cols - len(k) + 1];
+      for (uint32_t v = 1; v < tag_cols + 2; ++v) first[v] += first[v - 1];
+      for (uint32_t k : lv) sorted[first[tag_cols - len(k)]++] = k;
+      lv.swap(sorted);
+    }
+    for (uint32_t k : lv) ++cnt[std::min<uint32_t>(S[k], 33)];
     uint32_t at = 0;
-    std::vector<uint32_t> start(34, 0);
     for (int v = 33; v >= 1; --v) {
       start[v] = at;
       at += cnt[v];
     }
-    for (uint32_t k : live) sorted[start[std::min<uint32_t>(S[k], 33)]++] = k;
-    const uint32_t n_long = cnt[33];
-    std::stable_sort(sorted.begin(), sorted.begin() + n_long,
+    for (uint32_t k : lv) sorted[start[std::min<uint32_t>(S[k], 33)]++] = k;
+    std::stable_sort(sorted.begin(), sorted.begin() + cnt[33],
                      [&](uint32_t a, uint32_t b) { return S[a] > S[b]; });
-    live.swap(sorted);
-  }
-  std::vector<uint32_t> order;
-  std::vector<uint2> tasks;
-  order.reserve(live.size());
-  uint32_t open_start = 0, open_count = 0, open_free = 0, open_smax = 0;
-  auto close_tile = [&]() {
-    if (open_count) tasks.push_back(make_uint2(open_start, open_count | (open_smax << 16)));
-    open_count = 0;
-  };
-  for (uint32_t k : live) {
-    if (S[k] > 32) {
-      tasks.push_back(make_uint2((uint32_t)order.size(), 1u | (S[k] << 16)));
+    const uint32_t mark = kind == kT28 ? kTag28 : 0u;
+    uint32_t open_start = 0, open_count = 0, open_free = 0, open_smax = 0;
+    auto close_tile = [&]() {
+      if (open_count) tasks.push_back(make_uint2(open_start, open_count | mark | (open_smax << 16)));
+      open_count = 0;
+    };
+    for (uint32_t k : sorted) {
+      if (S[k] > 32) {
+        tasks.push_back(make_uint2((uint32_t)order.size(), 1u | (S[k] << 16)));
+        order.push_back(k);
+        continue;
+      }
+      if (!open_count || S[k] > open_free) {
+        close_tile();
+        open_start = (uint32_t)order.size();
+        open_free = 32;
+        open_smax = S[k];
+      }
       order.push_back(k);
-      continue;
+      open_free -= S[k];
+      ++open_count;
     }
-    if (!open_count || S[k] > open_free) {
-      close_tile();
-      open_start = (uint32_t)order.size();
-      open_free = 32;
-      open_smax = S[k];
-    }
-    order.push_back(k);
-    open_free -= S[k];
-    ++open_count;
+    close_tile();
   }
-  close_tile();
+  const uint32_t n_full = (uint32_t)tasks.size() - n_tag;
   const uint32_t n_tasks = (uint32_t)tasks.size();
 
   // --- geometry and scratch: per warp passes x columns x 32 lanes of 8 B,
   // capped at 4 GiB in all
-  const size_t trace_words = (size_t)passes_max * mcols * 32;
-  if (trace_words * 8 > (1ull << 30))
+  if ((size_t)all_passes * all_cols * 32 * 8 > (1ull << 30))
     return terr(ESG_ERR_BAD_ARGUMENT,
-                "a job of %u stripes x %u columns needs over 1 GiB of trace per warp", passes_max * 32,
-                mcols);
-  int per_sm = 0;
+                "a job of %u stripes x %u columns needs over 1 GiB of trace per warp",
+                all_passes * 32, all_cols);
+  const size_t trace_words = (size_t)passes_max * mcols * 32;
   cudaSetDevice(P.device);
-  const void* fn = P.mode == ESG_MODE_LOCAL ? (const void*)k7_trace<true>
-                                            : (const void*)k7_trace<false>;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, kTThreads, 0) != cudaSuccess)
-    per_sm = 1;
-  uint64_t warps = std::min<uint64_t>((uint64_t)std::max(per_sm, 1) * P.sm_count * kTWarps,
-                                      std::max<uint32_t>(n_tasks, 1));
-  warps = std::min<uint64_t>(warps, std::max<uint64_t>(kTWarps, (4ull << 30) / (trace_words * 8)));
-  const uint64_t blocks = std::max<uint64_t>(1, (warps + kTWarps - 1) / kTWarps);
-  warps = blocks * kTWarps;
+  const bool local = P.mode == ESG_MODE_LOCAL;
+  const void* fn = local ? (const void*)k7_trace<true> : (const void*)k7_trace<false>;
+  const void* tag_fn = local ? (const void*)k7_tags<true> : (const void*)k7_tags<false>;
+  auto grid = [&](const void* f, uint32_t n, size_t warp_bytes, uint64_t most) -> uint64_t {
+    if (!n) return 0;
+    int per_sm = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, f, kTThreads, 0) != cudaSuccess)
+      per_sm = 1;
+    uint64_t w = std::min<uint64_t>((uint64_t)std::max(per_sm, 1) * P.sm_count * kTWarps, n);
+    w = std::min<uint64_t>(w, std::max<uint64_t>(kTWarps, most / warp_bytes));
+    return (w + kTWarps - 1) / kTWarps;
+  };
+  const uint32_t tag_steps = tag_cols + tag_stripes - 1;
+  const size_t tag_bytes = (size_t)tag_steps * 128 * sizeof(uint4);
+  const uint64_t blocks = grid(fn, n_full, trace_words * 8, 4ull << 30);
+  const uint64_t tag_blocks = grid(tag_fn, n_tag, tag_bytes, kTagBytes);
+  const uint64_t warps = blocks * kTWarps;
+  const size_t scratch = warps * trace_words * 8;
 
   const size_t nj = std::max<uint32_t>(n_jobs, 1);
   const size_t sizes[] = {
@@ -459,11 +850,11 @@ esg_status align_impl(esg_scorer* sc, const uint8_t* d_codes, const uint64_t* d_
       align256(nj * 8),                          // job_at
       align256(std::max<size_t>(order.size(), 1) * 4),
       align256(std::max<uint32_t>(n_tasks, 1) * 8),
-      align256(4),                               // task counter
+      align256(8),                               // task counters
       align256(nj * 16),                         // res
       align256(nj * 16),                         // res2
       align256(std::max<uint64_t>(staging, 1) * 4),
-      align256(warps * trace_words * 8),
+      align256(scratch),
       align256(warps * (size_t)mcols * 8),
       align256(nj * 8),                          // dst
   };
@@ -499,7 +890,7 @@ esg_status align_impl(esg_scorer* sc, const uint8_t* d_codes, const uint64_t* d_
     TCUDA(cudaMemcpyAsync(d_order, order.data(), order.size() * 4, cudaMemcpyHostToDevice, st));
   if (n_tasks)
     TCUDA(cudaMemcpyAsync(d_tasks, tasks.data(), n_tasks * 8, cudaMemcpyHostToDevice, st));
-  TCUDA(cudaMemsetAsync(d_counter, 0, 4, st));
+  TCUDA(cudaMemsetAsync(d_counter, 0, 8, st));
   TCUDA(cudaMemsetAsync(d_res, 0, nj * 16, st));   // empty jobs stay all zero
   TCUDA(cudaMemsetAsync(d_res2, 0, nj * 16, st));
   if (n_tasks) {
@@ -515,8 +906,6 @@ esg_status align_impl(esg_scorer* sc, const uint8_t* d_codes, const uint64_t* d_
     K.job_at = d_job_at;
     K.order = d_order;
     K.tasks = d_tasks;
-    K.n_tasks = n_tasks;
-    K.task_counter = d_counter;
     K.trace = d_trace;
     K.trace_words = trace_words;
     K.mcols = mcols;
@@ -528,8 +917,28 @@ esg_status align_impl(esg_scorer* sc, const uint8_t* d_codes, const uint64_t* d_
     K.res = d_res;
     K.res2 = d_res2;
     K.ops = d_staging;
-    void* args[] = {&K};
-    TCUDA(cudaLaunchKernel(fn, dim3((unsigned)blocks), dim3(kTThreads), args, 0, st));
+    if (n_tag) {
+      // its scratch comes from a pool the device's scorers share: mapping it
+      // anew for each of them took longer (25 ms for 0.6 GB) than the tracing
+      uint4* d_tags = nullptr;
+      TCUDA(cudaMallocFromPoolAsync((void**)&d_tags, tag_blocks * kTWarps * tag_bytes,
+                                    esg_internal_trace_pool(P.device, kTagBytes, P.pool), st));
+      K7TagParams T{K, d_tags, tag_steps, 1};
+      T.J.n_tasks = n_tag;
+      T.J.task_counter = d_counter;
+      void* args[] = {&T};
+      const cudaError_t e =
+          cudaLaunchKernel(tag_fn, dim3((unsigned)tag_blocks), dim3(kTThreads), args, 0, st);
+      cudaFreeAsync(d_tags, st);
+      TCUDA(e);
+    }
+    if (n_full) {
+      K.tasks = d_tasks + n_tag;
+      K.n_tasks = n_full;
+      K.task_counter = d_counter + 1;
+      void* args[] = {&K};
+      TCUDA(cudaLaunchKernel(fn, dim3((unsigned)blocks), dim3(kTThreads), args, 0, st));
+    }
   }
   // --- results, then the words packed into the caller's layout
   std::vector<int4> res(nj), res2(nj);

@@ -153,3 +153,31 @@ def test_trace_pair_winners_on_trimmed_mates(oracle):
         pi = jobs[p][0] // 2
         assert int(al.records[p]["score"]) + int(al.records[p + 1]["score"]) == \
             int(got.pairs["best"][pi])
+
+
+@pytest.mark.parametrize("mode", [Mode.LOCAL, Mode.SEMIGLOBAL])
+def test_trace_tagged_values_at_their_edges(oracle, mode):
+    """Read lengths around a stripe of 28 and 32 rows, the last length and the
+    last reference on the tagged values and the first past them, references
+    of one base, gaps of hundreds of bases, free gap extension (ties between
+    extending and opening), wildcards, and a scheme whose longer jobs pass the
+    bound on 16-bit scores."""
+    rng = np.random.default_rng(0x7A6)
+    panel = [rng.integers(0, 5 if m == 300 else 4, m).astype(np.uint8)
+             for m in (1, 33, 300, 1200, 1700, 1701)]
+    reads = []
+    for k, n in enumerate((1, 27, 28, 29, 32, 33, 56, 57, 64, 224, 225, 896, 1023, 1024, 1025)):
+        ref = panel[2 + k % 4]
+        cut = np.concatenate([ref[:n - n // 2], ref[-(n // 2):]]) if n > 1 else ref[:1]
+        r = np.resize(cut, n).copy()  # both ends of a reference: one long deletion
+        if k % 3 == 1:
+            r[n // 3:n // 2] = rng.integers(0, 4, n // 2 - n // 3)
+        reads.append(r.astype(np.uint8))
+    big = panel[3]
+    reads.append(np.concatenate([big[:300], rng.integers(0, 4, 200).astype(np.uint8), big[300:600]]))
+    jobs = [(i, r, v) for i in range(len(reads)) for r in range(len(panel)) for v in (0, 1)
+            if v == 0 or i % 4 == 0]
+    for scoring in ((2, -1, -10, -1), (3, -2, -4, 0), (2, -1, 0, 0), (60, -40, -90, -2)):
+        with GpuScorer(panel, Scoring(*scoring), mode) as g:
+            check(oracle, g, reads, panel, jobs, scoring, mode == Mode.LOCAL,
+                  f"tags {mode.label} {scoring}")
