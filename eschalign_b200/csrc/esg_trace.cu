@@ -345,8 +345,8 @@ __global__ void __launch_bounds__(kTThreads) k7_trace(const K7Params P) {
 // bytes, rows 8 q .. 8 q + 7 of the stripe.
 // What bounds it: issue slots (11 instructions a cell) and the walk's loads;
 // the scratch (2 bytes a cell) is written once, 3.5 GB of DRAM traffic here.
-// 100 000 jobs of ~110 nt x 70-180 nt: 2.9 -> 1.2 ms semi-global, 3.7 -> 1.2
-// local.
+// 100 000 jobs of ~110 nt x 70-180 nt: 2.9 -> 1.4 ms semi-global, 3.7 -> 1.4
+// local (on 330 CTAs; 1.2 on 444, whose scratch is 0.77 GB).
 constexpr int kTagRows = 1024;    // longest read
 constexpr int kTagCols = 1700;    // longest reference: 592 warps' scratch in kTagBytes
 constexpr uint64_t kTagBytes = 2ull << 30;
@@ -833,13 +833,20 @@ esg_status align_impl(esg_scorer* sc, const uint8_t* d_codes, const uint64_t* d_
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, f, kTThreads, 0) != cudaSuccess)
       per_sm = 1;
     uint64_t w = std::min<uint64_t>((uint64_t)std::max(per_sm, 1) * P.sm_count * kTWarps, n);
-    w = std::min<uint64_t>(w, std::max<uint64_t>(kTWarps, most / warp_bytes));
+    w = std::min<uint64_t>(w, std::max<uint64_t>(kTWarps, most / warp_bytes / kTWarps * kTWarps));
     return (w + kTWarps - 1) / kTWarps;
   };
   const uint32_t tag_steps = tag_cols + tag_stripes - 1;
   const size_t tag_bytes = (size_t)tag_steps * 128 * sizeof(uint4);
   const uint64_t blocks = grid(fn, n_full, trace_words * 8, 4ull << 30);
-  const uint64_t tag_blocks = grid(tag_fn, n_tag, tag_bytes, kTagBytes);
+  // k7_tags' scratch: the least of 512 MiB, 1 and 2 GiB that holds four warps
+  // an SM, and all of it once a call needs half (what the shared pool keeps
+  // then fits the next call, whose jobs need a little more)
+  uint64_t tag_room = kTagBytes / 4;
+  while (tag_room < kTagBytes && tag_room / tag_bytes < 4ull * P.sm_count) tag_room *= 2;
+  const uint64_t tag_blocks = grid(tag_fn, n_tag, tag_bytes, tag_room);
+  const uint64_t tag_need = tag_blocks * kTWarps * tag_bytes;
+  const uint64_t tag_alloc = tag_need > tag_room / 2 ? std::max(tag_need, tag_room) : tag_need;
   const uint64_t warps = blocks * kTWarps;
   const size_t scratch = warps * trace_words * 8;
 
@@ -921,7 +928,7 @@ esg_status align_impl(esg_scorer* sc, const uint8_t* d_codes, const uint64_t* d_
       // its scratch comes from a pool the device's scorers share: mapping it
       // anew for each of them took longer (25 ms for 0.6 GB) than the tracing
       uint4* d_tags = nullptr;
-      TCUDA(cudaMallocFromPoolAsync((void**)&d_tags, tag_blocks * kTWarps * tag_bytes,
+      TCUDA(cudaMallocFromPoolAsync((void**)&d_tags, tag_alloc,
                                     esg_internal_trace_pool(P.device, kTagBytes, P.pool), st));
       K7TagParams T{K, d_tags, tag_steps, 1};
       T.J.n_tasks = n_tag;
