@@ -275,7 +275,7 @@ def encode_pairs(batch: BamBatch, mapping, ref_names, adapter_bases=None,
 class BamWriter:
     """esg_bam_writer_*: header, then pushed chunks in sequence order (or in
     coordinate order at close), BGZF-compressed on host threads, or on
-    `device` (esg_bam_writer_use_device: one warp per block)."""
+    `device` (esg_bam_writer_use_device: one CTA per block)."""
 
     def __init__(self, path: str, header_text: bytes, ref_names, ref_lens,
                  sort_coordinate: bool = False, threads: int = 0, device: int | None = None):

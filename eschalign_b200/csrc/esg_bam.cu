@@ -1565,7 +1565,7 @@ static esg_status device_start(esg_bam_writer* w, size_t whole) {
     e = cudaStreamCreateWithPriority(&D.stream, cudaStreamNonBlocking, greatest);
     if (e == cudaSuccess)
       e = cudaFuncSetAttribute(dz::k_bgzf_deflate, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int)sizeof(dz::BlockState));
+                               (int)sizeof(dz::DevState));
     if (e != cudaSuccess) return cuda_fail(w, e, "creating the stream");
   }
   if (nb > D.cap) {
@@ -1591,7 +1591,7 @@ static esg_status device_start(esg_bam_writer* w, size_t whole) {
   }
   e = cudaMemcpyAsync(D.d_in, w->pending.data(), whole, cudaMemcpyHostToDevice, D.stream);
   if (e != cudaSuccess) return cuda_fail(w, e, "uploading");
-  dz::k_bgzf_deflate<<<(unsigned)nb, dz::kLanes, sizeof(dz::BlockState), D.stream>>>(
+  dz::k_bgzf_deflate<<<(unsigned)nb, dz::kDefThreads, sizeof(dz::DevState), D.stream>>>(
       D.d_in, whole, D.d_tok, D.d_out, D.d_len);
   e = cudaGetLastError();
   if (e == cudaSuccess)

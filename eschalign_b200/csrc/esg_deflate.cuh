@@ -1,31 +1,28 @@
-// BGZF block compression on the device: one warp per BGZF block, DEFLATE
+// BGZF block compression on the device: one CTA per BGZF block, DEFLATE
 // (RFC 1951) with one dynamic-Huffman block per BGZF block.
 //
 // The BGZF writer of the BAM stage cuts the record stream into blocks of at
 // most 0xff00 bytes and deflates each on its own; the host cores at zlib's
 // level 6 spend about 11 core-seconds per million 150-nt records on it.
-// Blocks are independent, so here each one is a CTA of one warp:
-//   1. each lane runs a greedy LZ77 over its 2040-byte stripe of the block
-//      (a private 2048-entry table of the last position per 4-byte hash, primed
-//      with the 512 bytes before the stripe, matches clipped at the stripe's
-//      end) and writes its tokens to global scratch, counting the literal /
-//      length and distance symbols in shared memory;
-//   2. lane 0 builds the length-limited Huffman codes (two-queue Huffman on
-//      the sorted frequencies, lengths folded to 15 bits by moving leaves
-//      down until Kraft's sum is one) and the block header (code lengths
-//      run-length coded with symbols 16/17/18, RFC 1951 section 3.2.7);
-//   3. each lane sums its tokens' bits, a warp scan gives every lane its
-//      bit offset, and the lanes write their bits into the block's output
-//      slot (whole words with plain stores, the two shared edge words with
-//      atomicOr).
+// Blocks are independent.  Each one's steps:
+//   1. a greedy LZ77 over each of 32 stripes of 2040 bytes (a private
+//      2048-entry table of the last position per 4-byte hash, primed with the
+//      512 bytes before the stripe, matches clipped at the stripe's end) gives
+//      the tokens and counts the literal / length and distance symbols;
+//   2. the length-limited Huffman codes (two-queue Huffman on the sorted
+//      frequencies, lengths folded to 15 bits by moving leaves down until
+//      Kraft's sum is one) and the block header (code lengths run-length coded
+//      with symbols 16/17/18, RFC 1951 section 3.2.7);
+//   3. each stripe's tokens' bits, at the offset a scan over the stripes gives.
 // A block whose code would not be smaller than a stored block is reported
 // as such (length kStored) and the host writes it stored.  The output is a
 // valid DEFLATE stream that any inflater reads; it is not byte-identical to
 // zlib's (the records it holds are).
 //
-// Every function below except the kernel is __host__ __device__: the host
-// build runs the same steps lane by lane (esg_bgzf_deflate_host), which
-// is how the CPU tests check them against zlib's inflate.
+// The steps are written out stripe by stripe for the host
+// (esg_bgzf_deflate_host), which is how the CPU tests check them against
+// zlib's inflate; the kernel runs them in parallel to the same bytes, which is
+// how the GPU tests check it.
 #pragma once
 #include <stddef.h>
 #include <stdint.h>
@@ -56,8 +53,7 @@ constexpr uint32_t kMaxSyms = 288;
 constexpr uint32_t kTokensPerBlock = kLanes * kLaneBytes;
 constexpr uint32_t kMatchFlag = 0x80000000u;
 
-// Shared state of one block.  The per-lane hash tables and the staged input
-// dominate (128 KiB + 64 KiB): one CTA per SM.
+// The host steps' state of one block.
 struct BlockState {
   uint8_t in[kBlockIn];
   uint16_t table[kLanes * kHashSize];
@@ -76,7 +72,7 @@ struct BlockState {
   uint32_t n_lit, n_dist, n_cl;
   uint32_t header_bits;
   uint32_t lane_bits[kLanes];
-  // Huffman scratch (lane 0)
+  // Huffman scratch
   uint32_t h_weight[2 * kMaxSyms];
   uint16_t h_parent[2 * kMaxSyms];
   uint16_t h_sorted[kMaxSyms];
@@ -140,7 +136,7 @@ ESG_DHD inline void count(uint32_t* c) {
 #endif
 }
 
-// Step 1 for one lane: greedy LZ77 over the lane's stripe of the block
+// Step 1 for one stripe: greedy LZ77 over the lane's stripe of the block
 // `d[0, n)`; tokens (a byte, or kMatchFlag | (L - 3) << 15 | (D - 1)) go to
 // tok[k * stride].  Returns the token count (at most kLaneBytes).
 ESG_DHD inline uint32_t lz_stripe(const uint8_t* d, uint32_t n, uint32_t lane, uint16_t* tab,
@@ -304,7 +300,7 @@ ESG_DHD inline uint32_t cl_extra_bits(uint32_t sym) {
   return sym == 16 ? 2u : sym == 17 ? 3u : sym == 18 ? 7u : 0u;
 }
 
-// Step 2 (lane 0): the codes and the header's items; S.header_bits is the
+// Step 2: the codes and the header's items; S.header_bits is the
 // header's length in bits (BFINAL, BTYPE, HLIT, HDIST, HCLEN, the
 // code-length code, the items).
 ESG_DHD inline void build_codes(BlockState& S) {
@@ -449,7 +445,7 @@ ESG_DHD inline void put_token(const BlockState& S, BitSink& o, uint32_t t) {
 
 namespace esg_deflate {
 
-// The steps of the kernel below, lane by lane on the host: `out` (kSlotBytes
+// The steps, stripe by stripe on the host: `out` (kSlotBytes
 // bytes, 4-byte aligned) receives the DEFLATE stream of d[0, n); returns its
 // length in bytes, or kStored.  Used by the CPU tests of the steps.
 inline uint32_t deflate_block_host(const uint8_t* d, uint32_t n, uint8_t* out, BlockState& S,
@@ -486,17 +482,326 @@ inline uint32_t deflate_block_host(const uint8_t* d, uint32_t n, uint8_t* out, B
 }
 
 #ifdef __CUDACC__
-// One CTA of one warp per BGZF block b: in[b * kBlockIn, ...) of n_in bytes
-// in all -> out[b * kSlotBytes / 4, ...) and out_len[b] (bytes, or
-// kStored).  tokens: kTokensPerBlock words of scratch per block.  Dynamic
-// shared memory: sizeof(BlockState).
-__global__ void __launch_bounds__(32) k_bgzf_deflate(const uint8_t* __restrict__ in,
-                                                      uint64_t n_in, uint32_t* __restrict__ tokens,
-                                                      uint32_t* __restrict__ out,
-                                                      uint32_t* __restrict__ out_len) {
+// ------------------------------------------------------------ the kernel
+// One CTA of 16 warps per BGZF block.  The steps above are sequential per
+// stripe only on the face of it:
+//   1. Every position before p has been entered into the stripe's table by
+//      the time p is looked up, whatever was matched, so p's candidate is the
+//      last earlier position of its hash.  A warp takes a stripe 32 positions
+//      at a time: candidates by a match over the warp and one table access,
+//      a ballot of the positions whose four bytes agree, then the greedy walk
+//      over that mask -- the literals up to the next match written together, a
+//      match's length compared 8 bytes a lane.
+//   2. The sort, the depths, the code lengths and the codes are a thread per
+//      symbol; one thread merges the two queues.
+//   3. A warp sums and writes its stripes' bits 32 tokens at a time, into
+//      shared memory, where the tables were.
+// The same tokens, frequencies, codes and bits as the steps give, byte for
+// byte.  One warp per block with a table and a stripe per lane, the codes by
+// one lane, took 4.5 ms a block whatever their number up to one per SM (a
+// serial chain: every step waited for shared memory); this takes
+// 0.36, and 134 blocks 0.39 (4.8 before).
+constexpr uint32_t kDefWarps = 16;
+constexpr uint32_t kDefThreads = kDefWarps * 32;
+constexpr uint32_t kDefFull = 0xffffffffu;
+
+struct DevHuff {  // one code: literal / length, distance or code-length symbols
+  uint32_t freq[kMaxSyms];
+  uint32_t w[2 * kMaxSyms];      // node weights, leaves by (weight, symbol) first
+  uint16_t par[2 * kMaxSyms];
+  uint16_t sorted[kMaxSyms];
+  uint8_t len[kMaxSyms];
+  uint16_t code[kMaxSyms];
+  uint32_t bl[32];
+  uint32_t m, maxd;
+};
+
+struct DevState {
+  uint8_t in[kBlockIn];
+  union {
+    uint16_t table[kDefWarps * kHashSize];
+    uint32_t out[kSlotBytes / 4];
+  };
+  DevHuff lit, dist, cl;
+  uint16_t items[kNumLit + kNumDist];
+  uint32_t n_items, n_lit, n_dist, n_cl, header_bits;
+  uint32_t n_tok[kLanes], bits[kLanes], start[kLanes + 1];
+};
+
+// Four bytes of the block at any position (may read past the block, never
+// past the state).
+__device__ __forceinline__ uint32_t load4(const uint8_t* in, uint32_t p) {
+  const uint32_t* w = reinterpret_cast<const uint32_t*>(in) + (p >> 2);
+  return __funnelshift_r(w[0], w[1], (p & 3u) * 8u);
+}
+
+// Step 1, one warp: the tokens of stripe `st`.
+__device__ inline uint32_t lz_stripe_warp(DevState& S, uint32_t n, uint32_t st, uint16_t* tab,
+                                          uint32_t* tok, int lane) {
+  const uint32_t s = st * kLaneBytes;
+  if (s >= n) return 0;
+  const uint32_t e = s + kLaneBytes < n ? s + kLaneBytes : n;
+  for (uint32_t i = lane; i < kHashSize / 2; i += 32)
+    reinterpret_cast<uint32_t*>(tab)[i] = 0xffffffffu;
+  __syncwarp();
+  uint32_t nt = 0, pos = s;  // pos: the walk's next position
+  for (uint32_t p0 = s > kLookback ? s - kLookback : 0; p0 < e; p0 += 32) {
+    const uint32_t q = p0 + lane;
+    const bool in = q + 4 <= n && q < e;
+    const uint32_t x = in ? load4(S.in, q) : 0u;
+    const uint32_t h = (x * 2654435761u) >> (32 - kHashBits);
+    const uint32_t peers = __match_any_sync(kDefFull, in ? h : kHashSize + (uint32_t)lane);
+    const uint32_t before = peers & ((1u << lane) - 1u);
+    uint32_t c = kEmpty;
+    if (in) c = before ? p0 + (31u - (uint32_t)__clz((int)before)) : tab[h];
+    __syncwarp();
+    if (in && (peers >> lane) == 1u) tab[h] = (uint16_t)q;
+    __syncwarp();
+    if (p0 + 32 <= pos) continue;  // priming, or inside a match
+    const bool ok = q >= s && q + kMinMatch <= e && c != kEmpty && load4(S.in, c) == x;
+    const uint32_t mask = __ballot_sync(kDefFull, ok);
+    const uint32_t end = p0 + 32 < e ? p0 + 32 : e;
+    while (pos < end) {
+      const uint32_t left = mask & (kDefFull << (pos - p0));
+      const uint32_t p = left ? p0 + (uint32_t)__ffs((int)left) - 1u : end;
+      if (q >= pos && q < p) {  // literals up to the match
+        const uint32_t v = S.in[q];
+        tok[nt + (q - pos)] = v;
+        atomicAdd(&S.lit.freq[v], 1u);
+      }
+      nt += p - pos;
+      pos = p;
+      if (!left) break;
+      const uint32_t cp = __shfl_sync(kDefFull, c, (int)(p - p0));
+      const uint32_t lim = e - p < kMaxMatch ? e - p : kMaxMatch;
+      const uint32_t o = kMinMatch + 8 * (uint32_t)lane;
+      uint32_t same = 0;  // equal bytes from o on, of 8
+      if (o < lim) {
+        const uint32_t d0 = load4(S.in, p + o) ^ load4(S.in, cp + o);
+        const uint32_t d1 = load4(S.in, p + o + 4) ^ load4(S.in, cp + o + 4);
+        same = d0 ? (uint32_t)(__ffs((int)d0) - 1) / 8 : d1 ? 4 + (uint32_t)(__ffs((int)d1) - 1) / 8 : 8;
+      }
+      const uint32_t differ = __ballot_sync(kDefFull, same < 8);
+      const int at = differ ? __ffs((int)differ) - 1 : 31;
+      uint32_t L = kMinMatch + 8 * (uint32_t)at + __shfl_sync(kDefFull, same, at);
+      L = L < lim ? L : lim;
+      if (lane == 0) {
+        tok[nt] = kMatchFlag | (L - 3) << 15 | (p - cp - 1);
+        uint32_t sym, nx, xv;
+        length_symbol(L, sym, nx, xv);
+        atomicAdd(&S.lit.freq[sym], 1u);
+        distance_symbol(p - cp, sym, nx, xv);
+        atomicAdd(&S.dist.freq[sym], 1u);
+      }
+      ++nt;
+      pos = p + L;
+    }
+  }
+  return nt;
+}
+
+// Code lengths (at most `limit` bits) and codes of one or two alphabets at
+// once: thread i < n of a group of threads takes symbol i of H (H null: no
+// symbol).  Called by the whole CTA.
+__device__ inline void codes_block(DevHuff* H, uint32_t i, uint32_t n, uint32_t limit) {
+  const bool on = H && i < n;
+  if (on && i == 0) {
+    // fewer than two symbols in use: the first unused ones get weight 1
+    uint32_t m = 0;
+    for (uint32_t k = 0; k < n && m < 2; ++k) m += H->freq[k] != 0;
+    for (uint32_t k = 0; m < 2 && k < n; ++k)
+      if (!H->freq[k]) {
+        H->freq[k] = 1;
+        ++m;
+      }
+    H->m = 0;
+    H->maxd = 0;
+  }
+  if (on && i < 32) H->bl[i] = 0;
+  if (on && n < 32 && i == 0)
+    for (uint32_t k = n; k < 32; ++k) H->bl[k] = 0;
+  __syncthreads();
+  const uint32_t wi = on ? H->freq[i] : 0u;
+  uint32_t rank = 0;
+  if (wi) {
+    for (uint32_t k = 0; k < n; ++k) {
+      const uint32_t wk = H->freq[k];
+      rank += wk && (wk < wi || (wk == wi && k < i));
+    }
+    H->sorted[rank] = (uint16_t)i;
+    H->w[rank] = wi;
+    atomicAdd(&H->m, 1u);
+  }
+  __syncthreads();
+  if (on && i == 0) {
+    // two-queue Huffman: leaves 0..m-1 by weight, internal nodes m..2m-2 are
+    // made in nondecreasing weight order
+    const uint32_t m = H->m;
+    uint32_t li = 0, ii = m, nx = m;
+    uint32_t wl = H->w[0], wn = 0;
+    for (uint32_t k = 0; k + 1 < m; ++k) {
+      uint32_t sum = 0;
+#pragma unroll
+      for (int t = 0; t < 2; ++t) {
+        if (li < m && (ii >= nx || wl <= wn)) {
+          H->par[li] = (uint16_t)nx;
+          sum += wl;
+          ++li;
+          wl = li < m ? H->w[li] : 0u;
+        } else {
+          H->par[ii] = (uint16_t)nx;
+          sum += wn;
+          ++ii;
+          wn = ii < nx ? H->w[ii] : 0u;
+        }
+      }
+      H->w[nx] = sum;
+      if (ii == nx) wn = sum;
+      ++nx;
+    }
+  }
+  __syncthreads();
+  if (wi) {
+    const uint32_t root = 2 * H->m - 2;
+    uint32_t d = 0;
+    for (uint32_t v = rank; v != root; v = H->par[v]) ++d;
+    d = d < 31 ? d : 31;
+    atomicAdd(&H->bl[d], 1u);
+    atomicMax(&H->maxd, d);
+  }
+  __syncthreads();
+  if (on && i == 0 && H->maxd > limit) {
+    // fold lengths above the limit into it, then move leaves one level down
+    // until Kraft's sum is exactly one
+    uint32_t* bl = H->bl;
+    for (uint32_t L = limit + 1; L <= H->maxd; ++L) {
+      bl[limit] += bl[L];
+      bl[L] = 0;
+    }
+    uint64_t total = 0;
+    for (uint32_t L = 1; L <= limit; ++L) total += (uint64_t)bl[L] << (limit - L);
+    while (total > (1ull << limit)) {
+      --bl[limit];
+      for (uint32_t L = limit - 1; L > 0; --L)
+        if (bl[L]) {
+          --bl[L];
+          bl[L + 1] += 2;
+          break;
+        }
+      --total;
+    }
+    H->maxd = limit;
+  }
+  __syncthreads();
+  uint32_t L = 0;
+  if (wi) {  // the lightest leaves take the longest codes
+    uint32_t seen = 0;
+    for (L = H->maxd; L > 1; --L) {
+      seen += H->bl[L];
+      if (rank < seen) break;
+    }
+  }
+  if (on) H->len[i] = (uint8_t)L;
+  __syncthreads();
+  if (on) {
+    uint32_t v = 0;
+    if (L) {
+      for (uint32_t b = 1; b <= L; ++b) v = (v + (b > 1 ? H->bl[b - 1] : 0u)) << 1;
+      for (uint32_t k = 0; k < i; ++k) v += H->len[k] == L;
+      v = __brev(v) >> (32 - L);
+    }
+    H->code[i] = (uint16_t)v;
+  }
+  __syncthreads();
+}
+
+// Step 2, after the codes of literals / lengths and distances: the header's
+// run-length items and their symbols' frequencies (one thread).
+__device__ inline void header_items(DevState& S) {
+  uint32_t nl = kNumLit, nd = kNumDist;
+  while (nl > 257 && !S.lit.len[nl - 1]) --nl;
+  while (nd > 1 && !S.dist.len[nd - 1]) --nd;
+  S.n_lit = nl;
+  S.n_dist = nd;
+  auto at = [&](uint32_t i) -> uint32_t { return i < nl ? S.lit.len[i] : S.dist.len[i - nl]; };
+  const uint32_t total = nl + nd;
+  for (uint32_t i = 0; i < kNumCl; ++i) S.cl.freq[i] = 0;
+  uint32_t ni = 0;
+  auto item = [&](uint32_t sym, uint32_t xv) {
+    S.items[ni++] = (uint16_t)(sym << 8 | xv);
+    ++S.cl.freq[sym];
+  };
+  for (uint32_t i = 0; i < total;) {
+    const uint32_t cur = at(i);
+    uint32_t run = 1;
+    while (i + run < total && at(i + run) == cur) ++run;
+    i += run;
+    if (cur == 0) {
+      while (run >= 11) {
+        const uint32_t r = run < 138 ? run : 138;
+        item(18, r - 11);
+        run -= r;
+      }
+      if (run >= 3) {
+        item(17, run - 3);
+        run = 0;
+      }
+      while (run--) item(0, 0);
+    } else {
+      item(cur, 0);
+      --run;
+      while (run >= 3) {
+        const uint32_t r = run < 6 ? run : 6;
+        item(16, r - 3);
+        run -= r;
+      }
+      while (run--) item(cur, 0);
+    }
+  }
+  S.n_items = ni;
+}
+
+// A token's bits, LSB first, and their number (at most 48).
+__device__ __forceinline__ uint64_t token_code(const DevState& S, uint32_t t, uint32_t& nb) {
+  if (!(t & kMatchFlag)) {
+    nb = S.lit.len[t];
+    return S.lit.code[t];
+  }
+  uint32_t sym, nx, xv;
+  length_symbol(((t >> 15) & 0xff) + 3, sym, nx, xv);
+  uint64_t v = S.lit.code[sym];
+  nb = S.lit.len[sym];
+  v |= (uint64_t)xv << nb;
+  nb += nx;
+  distance_symbol((t & 0x7fff) + 1, sym, nx, xv);
+  v |= (uint64_t)S.dist.code[sym] << nb;
+  nb += S.dist.len[sym];
+  v |= (uint64_t)xv << nb;
+  nb += nx;
+  return v;
+}
+
+__device__ __forceinline__ void put_bits(uint32_t* out, uint32_t bit, uint64_t v) {
+  const uint32_t w = bit >> 5, sh = bit & 31u;
+  const uint64_t lo = v << sh;
+  if ((uint32_t)lo) atomicOr(out + w, (uint32_t)lo);
+  if ((uint32_t)(lo >> 32)) atomicOr(out + w + 1, (uint32_t)(lo >> 32));
+  const uint32_t hi = sh ? (uint32_t)(v >> (64u - sh)) : 0u;
+  if (hi) atomicOr(out + w + 2, hi);
+}
+
+// Block b of the input: in[b * kBlockIn, ...) of n_in bytes in all ->
+// out[b * kSlotBytes / 4, ...) and out_len[b] (bytes, or kStored).  tokens:
+// kTokensPerBlock words of scratch per block.  Dynamic shared memory:
+// sizeof(DevState).
+__global__ void __launch_bounds__(kDefThreads) k_bgzf_deflate(const uint8_t* __restrict__ in,
+                                                               uint64_t n_in, uint32_t* tokens,
+                                                               uint32_t* __restrict__ out,
+                                                               uint32_t* __restrict__ out_len) {
   extern __shared__ __align__(16) uint8_t smem[];
-  BlockState& S = *reinterpret_cast<BlockState*>(smem);
-  const uint32_t b = blockIdx.x, lane = threadIdx.x;
+  DevState& S = *reinterpret_cast<DevState*>(smem);
+  const uint32_t b = blockIdx.x, tid = threadIdx.x, wib = tid >> 5;
+  const int lane = (int)(tid & 31u);
   const uint64_t base = (uint64_t)b * kBlockIn;
   if (base >= n_in) return;
   const uint32_t n = (uint32_t)(n_in - base < kBlockIn ? n_in - base : kBlockIn);
@@ -504,41 +809,110 @@ __global__ void __launch_bounds__(32) k_bgzf_deflate(const uint8_t* __restrict__
   // 16-byte aligned when `in` does)
   const uint4* src = reinterpret_cast<const uint4*>(in + base);
   uint4* dst = reinterpret_cast<uint4*>(S.in);
-  for (uint32_t i = lane; i < n / 16; i += kLanes) dst[i] = src[i];
-  for (uint32_t i = n / 16 * 16 + lane; i < n; i += kLanes) S.in[i] = in[base + i];
-  for (uint32_t i = lane; i < kMaxSyms; i += kLanes) S.lit_freq[i] = 0;
-  S.dist_freq[lane] = 0;
-  __syncwarp();
-  uint32_t* tok = tokens + (size_t)b * kTokensPerBlock + lane;
-  const uint32_t nt = lz_stripe(S.in, n, lane, S.table + lane * kHashSize, tok, kLanes,
-                                S.lit_freq, S.dist_freq);
-  __syncwarp();
-  if (lane == 0) build_codes(S);
-  __syncwarp();
-  uint32_t bits = lane == 0 ? S.header_bits : 0;
-  for (uint32_t k = 0; k < nt; ++k) bits += token_bits(S, tok[(size_t)k * kLanes]);
-  if (lane == kLanes - 1) bits += S.lit_len[256];
-  uint32_t incl = bits;
-  for (uint32_t dd = 1; dd < kLanes; dd <<= 1) {
-    const uint32_t v = __shfl_up_sync(0xffffffffu, incl, dd);
-    if (lane >= dd) incl += v;
+  for (uint32_t i = tid; i < n / 16; i += kDefThreads) dst[i] = src[i];
+  for (uint32_t i = n / 16 * 16 + tid; i < n; i += kDefThreads) S.in[i] = in[base + i];
+  for (uint32_t i = tid; i < kMaxSyms; i += kDefThreads) S.lit.freq[i] = S.dist.freq[i] = 0;
+  __syncthreads();
+  uint32_t* tok = tokens + (size_t)b * kTokensPerBlock;
+  for (uint32_t st = wib; st < kLanes; st += kDefWarps) {
+    const uint32_t nt = lz_stripe_warp(S, n, st, S.table + wib * kHashSize,
+                                       tok + st * kLaneBytes, lane);
+    if (lane == 0) S.n_tok[st] = nt;
   }
-  const uint32_t total = __shfl_sync(0xffffffffu, incl, kLanes - 1);
-  const uint32_t bytes = (total + 7) / 8;
+  __syncthreads();
+  if (tid == 0) S.lit.freq[256] += 1;  // end of block
+  __syncthreads();
+  {
+    const bool d = tid >= 480;  // the last warp: distances
+    codes_block(tid < kNumLit ? &S.lit : d ? &S.dist : nullptr, d ? tid - 480 : tid,
+                d ? kNumDist : kNumLit, 15);
+  }
+  if (tid == 0) header_items(S);
+  __syncthreads();
+  codes_block(tid < kNumCl ? &S.cl : nullptr, tid, kNumCl, 7);
+  if (tid == 0) {
+    uint32_t ncl = kNumCl;
+    while (ncl > 4 && !S.cl.len[cl_order(ncl - 1)]) --ncl;
+    S.n_cl = ncl;
+    uint32_t bits = 3 + 5 + 5 + 4 + 3 * ncl;
+    for (uint32_t k = 0; k < S.n_items; ++k) {
+      const uint32_t sym = S.items[k] >> 8;
+      bits += S.cl.len[sym] + cl_extra_bits(sym);
+    }
+    S.header_bits = bits;
+  }
+  // --- each stripe's bits
+  for (uint32_t st = wib; st < kLanes; st += kDefWarps) {
+    uint32_t bits = 0;
+    for (uint32_t k = lane; k < S.n_tok[st]; k += 32) {
+      uint32_t nb;
+      token_code(S, tok[st * kLaneBytes + k], nb);
+      bits += nb;
+    }
+    bits = __reduce_add_sync(kDefFull, bits);
+    if (lane == 0) S.bits[st] = bits;
+  }
+  __syncthreads();
+  if (wib == 0) {
+    uint32_t bits = S.bits[lane] + (lane == 0 ? S.header_bits : 0u) +
+                    (lane == (int)kLanes - 1 ? S.lit.len[256] : 0u);
+    uint32_t incl = bits;
+    for (int dd = 1; dd < 32; dd <<= 1) {
+      const uint32_t v = __shfl_up_sync(kDefFull, incl, dd);
+      if (lane >= dd) incl += v;
+    }
+    S.start[lane] = incl - bits;
+    if (lane == 31) S.start[kLanes] = incl;
+  }
+  __syncthreads();
+  const uint32_t total = S.start[kLanes], bytes = (total + 7) / 8;
   if (bytes > n + 5) {  // a stored block is no larger
-    if (lane == 0) out_len[b] = kStored;
+    if (tid == 0) out_len[b] = kStored;
     return;
   }
-  // bytes <= n + 5 <= kBlockIn + 5 < kSlotBytes: every word below is in the slot
+  // bytes <= n + 5 <= kBlockIn + 5 < kSlotBytes - 8: every word below is in S.out
+  const uint32_t words = (total + 31) / 32;
+  for (uint32_t i = tid; i < words; i += kDefThreads) S.out[i] = 0;
+  __syncthreads();
+  if (tid == 0) {
+    uint32_t at = 0;
+    auto put = [&](uint32_t v, uint32_t nb) {
+      put_bits(S.out, at, v);
+      at += nb;
+    };
+    put(1, 1);  // BFINAL
+    put(2, 2);  // BTYPE = 10: dynamic Huffman
+    put(S.n_lit - 257, 5);
+    put(S.n_dist - 1, 5);
+    put(S.n_cl - 4, 4);
+    for (uint32_t i = 0; i < S.n_cl; ++i) put(S.cl.len[cl_order(i)], 3);
+    for (uint32_t k = 0; k < S.n_items; ++k) {
+      const uint32_t sym = S.items[k] >> 8;
+      put(S.cl.code[sym], S.cl.len[sym]);
+      put(S.items[k] & 0xff, cl_extra_bits(sym));
+    }
+    put_bits(S.out, total - S.lit.len[256], S.lit.code[256]);
+  }
+  for (uint32_t st = wib; st < kLanes; st += kDefWarps) {
+    uint32_t at = S.start[st] + (st == 0 ? S.header_bits : 0u);
+    for (uint32_t k0 = 0; k0 < S.n_tok[st]; k0 += 32) {
+      const uint32_t k = k0 + lane;
+      uint32_t nb = 0;
+      uint64_t v = 0;
+      if (k < S.n_tok[st]) v = token_code(S, tok[st * kLaneBytes + k], nb);
+      uint32_t incl = nb;
+      for (int dd = 1; dd < 32; dd <<= 1) {
+        const uint32_t y = __shfl_up_sync(kDefFull, incl, dd);
+        if (lane >= dd) incl += y;
+      }
+      put_bits(S.out, at + incl - nb, v);
+      at += __shfl_sync(kDefFull, incl, 31);
+    }
+  }
+  __syncthreads();
   uint32_t* o = out + (size_t)b * (kSlotBytes / 4);
-  for (uint32_t i = lane; i < (total + 31) / 32; i += kLanes) o[i] = 0;
-  __syncwarp();
-  BitSink sink(o, incl - bits);
-  if (lane == 0) put_header(S, sink);
-  for (uint32_t k = 0; k < nt; ++k) put_token(S, sink, tok[(size_t)k * kLanes]);
-  if (lane == kLanes - 1) sink.put(S.lit_code[256], S.lit_len[256]);
-  sink.finish();
-  if (lane == 0) out_len[b] = bytes;
+  for (uint32_t i = tid; i < words; i += kDefThreads) o[i] = S.out[i];
+  if (tid == 0) out_len[b] = bytes;
 }
 #endif
 

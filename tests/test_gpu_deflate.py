@@ -123,3 +123,35 @@ def test_writer_switches_back_to_host(tmp_path):
 def test_bad_device_is_refused(tmp_path):
     with pytest.raises(Exception, match="no such device"):
         EB.BamWriter(str(tmp_path / "x.bam"), b"", ["r"], [1], device=4096)
+
+
+def _fibonacci_bytes(rng, n):
+    """Byte frequencies growing like Fibonacci numbers: code lengths past 15
+    bits before they are limited."""
+    f = [1, 1]
+    while sum(f) + f[-1] + f[-2] < n:
+        f.append(f[-1] + f[-2])
+    b = np.repeat(np.arange(1, len(f) + 1, dtype=np.uint8), f)
+    rng.shuffle(b)
+    return b.tobytes()
+
+
+@pytest.mark.parametrize("extra", [0, 1, 2, 3, 4, 5, 31, 2039, 2041, 65279])
+def test_edge_blocks_equal_the_host_steps(tmp_path, extra):
+    """Runs longer than the longest match and across stripes, periods around
+    the hash's four bytes, code lengths over the limit, a block of few
+    symbols, a last block of few bytes or one short of full."""
+    rng = np.random.default_rng(extra)
+    parts = [b"A" * 70_000, b"ACGT" * 9000, b"ACGTN" * 300 + b"B" * 263 + b"C" * 259,
+             _fibonacci_bytes(rng, 60_000), bytes(rng.integers(1, 4, 30_000, dtype=np.uint8))]
+    text = b"".join(parts)
+    text += b"xyz"[:extra % 4] + b"Q" * extra
+    pad = -(len(text) + 12 + 4 + 2 + 4) % 0xff00  # magic, lengths, one reference's entry
+    text += bytes(rng.integers(1, 255, pad, dtype=np.uint8)) + b"Q" * extra
+    path = str(tmp_path / "e.bam")
+    with EB.BamWriter(path, text, ["r"], [100], device=0):
+        pass
+    raw = gzip.decompress(open(path, "rb").read())
+    assert raw[8:8 + len(text)] == text
+    blocks, _ = _check_blocks(path)
+    assert blocks >= 3
