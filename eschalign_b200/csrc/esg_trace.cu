@@ -20,8 +20,8 @@
 // maximum in column-major order (local: every cell; semi-global: the last
 // row and the last column); a segmented shuffle reduction gives the job's
 // end cell, and the job's last lane follows the trace codes back
-// (scalar.rs:292-364), writing run-length CIGAR words.  k7_compact packs
-// the jobs' words into the caller's layout.
+// (scalar.rs:292-364), writing run-length CIGAR words.  k7_sums and
+// k7_pack put the jobs' words and records into the caller's layout.
 #include "../../include/eschalign_b200.h"
 #include "esg_internal.h"
 
@@ -675,14 +675,76 @@ __global__ void __launch_bounds__(kTThreads, 3) k7_tags(const K7TagParams P) {
   }
 }
 
-// Pack each job's CIGAR words from the staging into the caller's layout.
-__global__ void __launch_bounds__(256) k7_compact(const uint32_t* staging, const uint64_t* at,
-                                                  const uint64_t* dst, const int4* res2,
-                                                  uint32_t n_jobs, uint32_t* out) {
-  for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < n_jobs;
-       k += gridDim.x * blockDim.x) {
-    const uint32_t nr = (uint32_t)res2[k].y;
-    for (uint32_t w = 0; w < nr; ++w) out[dst[k] + w] = staging[at[k] + w];
+// ---------------------------------------------------------------- results
+// The caller's records and packed words, made on the device: each block's
+// words counted (k7_sums), then placed after the blocks before it (k7_pack).
+// Copying the kernels' results out and walking the jobs on the host for the
+// offsets, back up for the packing and again for the records took 1.3 ms a
+// 100 000 jobs.
+constexpr uint32_t kPackThreads = 256;
+constexpr uint32_t kPackJobs = 4 * kPackThreads;  // jobs a block
+
+__global__ void __launch_bounds__(kPackThreads) k7_sums(const int4* __restrict__ res2,
+                                                        uint32_t n_jobs,
+                                                        unsigned long long* __restrict__ sums) {
+  __shared__ unsigned long long sum;
+  if (threadIdx.x == 0) sum = 0;
+  __syncthreads();
+  uint32_t v = 0;
+  for (uint32_t i = threadIdx.x; i < kPackJobs; i += kPackThreads) {
+    const uint64_t k = (uint64_t)blockIdx.x * kPackJobs + i;
+    if (k < n_jobs) v += (uint32_t)res2[k].y;
+  }
+  v = __reduce_add_sync(kFullT, v);
+  if ((threadIdx.x & 31) == 0) atomicAdd(&sum, (unsigned long long)v);
+  __syncthreads();
+  if (threadIdx.x == 0) sums[blockIdx.x] = sum;
+}
+
+__global__ void __launch_bounds__(kPackThreads) k7_pack(const int4* __restrict__ res,
+                                                        const int4* __restrict__ res2,
+                                                        uint32_t n_jobs,
+                                                        const unsigned long long* __restrict__ sums,
+                                                        const uint32_t* __restrict__ staging,
+                                                        const uint64_t* __restrict__ at,
+                                                        esg_alignment* __restrict__ rec,
+                                                        uint32_t* __restrict__ words) {
+  __shared__ unsigned long long before;
+  __shared__ uint32_t warp_sum[kPackThreads / 32];
+  const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  if (threadIdx.x == 0) before = 0;
+  __syncthreads();
+  unsigned long long b = 0;
+  for (uint32_t i = threadIdx.x; i < blockIdx.x; i += kPackThreads) b += sums[i];
+  if (b) atomicAdd(&before, b);
+  const uint64_t k0 = (uint64_t)blockIdx.x * kPackJobs + 4 * threadIdx.x;
+  int4 r2[4];
+  uint32_t mine = 0;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    r2[i] = k0 + i < n_jobs ? res2[k0 + i] : make_int4(0, 0, 0, 0);
+    mine += (uint32_t)r2[i].y;
+  }
+  uint32_t incl = mine;
+#pragma unroll
+  for (int d = 1; d < 32; d <<= 1) {
+    const uint32_t v = __shfl_up_sync(kFullT, incl, d);
+    if (lane >= (uint32_t)d) incl += v;
+  }
+  if (lane == 31) warp_sum[warp] = incl;
+  __syncthreads();
+  unsigned long long o = before + incl - mine;
+  for (uint32_t w = 0; w < warp; ++w) o += warp_sum[w];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const uint64_t k = k0 + i;
+    if (k >= n_jobs) break;
+    const int4 r = res[k];
+    const uint32_t nr = (uint32_t)r2[i].y;
+    rec[k] = {r.x, (uint32_t)r.y, (uint32_t)r.z, (uint32_t)r.w, (uint32_t)r2[i].x, nr, o};
+    const uint32_t* src = staging + at[k];
+    for (uint32_t w = 0; w < nr; ++w) words[o + w] = src[w];
+    o += nr;
   }
 }
 
@@ -725,6 +787,8 @@ esg_status align_impl(esg_scorer* sc, const uint8_t* d_codes, const uint64_t* d_
   // jobs by kernel and stripe height: k7_tags on 28 and 32 rows, k7_trace
   enum { kT28, kT32, kFull, kKinds };
   std::vector<uint32_t> live[kKinds];
+  live[kT28].reserve(n_jobs);
+  live[kT32].reserve(n_jobs);
   const int64_t mm = std::max(std::abs(P.scoring.match_score), std::abs(P.scoring.mismatch)),
                 go = std::abs(P.scoring.gap_open), ge = std::abs(P.scoring.gap_extend);
   for (uint32_t k = 0; k < n_jobs; ++k) {
@@ -851,6 +915,7 @@ esg_status align_impl(esg_scorer* sc, const uint8_t* d_codes, const uint64_t* d_
   const size_t scratch = warps * trace_words * 8;
 
   const size_t nj = std::max<uint32_t>(n_jobs, 1);
+  const uint32_t pack_blocks = (uint32_t)((nj + kPackJobs - 1) / kPackJobs);
   const size_t sizes[] = {
       align256(nj * 4),                          // job_q
       align256(nj * 4),                          // job_slot
@@ -863,7 +928,8 @@ esg_status align_impl(esg_scorer* sc, const uint8_t* d_codes, const uint64_t* d_
       align256(std::max<uint64_t>(staging, 1) * 4),
       align256(scratch),
       align256(warps * (size_t)mcols * 8),
-      align256(nj * 8),                          // dst
+      align256(nj * sizeof(esg_alignment)),
+      align256(pack_blocks * 8),                 // words per block
   };
   size_t total = 0;
   for (size_t v : sizes) total += v;
@@ -887,7 +953,8 @@ esg_status align_impl(esg_scorer* sc, const uint8_t* d_codes, const uint64_t* d_
   uint32_t* d_staging = (uint32_t*)take(8);
   uint2* d_trace = (uint2*)take(9);
   uint2* d_colbuf = (uint2*)take(10);
-  uint64_t* d_dst = (uint64_t*)take(11);
+  esg_alignment* d_rec = (esg_alignment*)take(11);
+  unsigned long long* d_sums = (unsigned long long*)take(12);
   if (n_jobs) {
     TCUDA(cudaMemcpyAsync(d_job_q, job_q.data(), n_jobs * 4, cudaMemcpyHostToDevice, st));
     TCUDA(cudaMemcpyAsync(d_job_slot, job_slot.data(), n_jobs * 4, cudaMemcpyHostToDevice, st));
@@ -947,17 +1014,14 @@ esg_status align_impl(esg_scorer* sc, const uint8_t* d_codes, const uint64_t* d_
       TCUDA(cudaLaunchKernel(fn, dim3((unsigned)blocks), dim3(kTThreads), args, 0, st));
     }
   }
-  // --- results, then the words packed into the caller's layout
-  std::vector<int4> res(nj), res2(nj);
-  TCUDA(cudaMemcpyAsync(res.data(), d_res, nj * 16, cudaMemcpyDeviceToHost, st));
-  TCUDA(cudaMemcpyAsync(res2.data(), d_res2, nj * 16, cudaMemcpyDeviceToHost, st));
+  // --- how many words there are, then records and words packed
+  k7_sums<<<pack_blocks, kPackThreads, 0, st>>>(d_res2, n_jobs, d_sums);
+  TCUDA(cudaGetLastError());
+  std::vector<uint64_t> sums(pack_blocks);
+  TCUDA(cudaMemcpyAsync(sums.data(), d_sums, pack_blocks * 8, cudaMemcpyDeviceToHost, st));
   TCUDA(cudaStreamSynchronize(st));
-  std::vector<uint64_t> dst(nj, 0);
   uint64_t need = 0;
-  for (uint32_t k = 0; k < n_jobs; ++k) {
-    dst[k] = need;
-    need += (uint32_t)res2[k].y;
-  }
+  for (uint64_t v : sums) need += v;
   if (ops_needed) *ops_needed = need;
   if (grow) {
     grow->resize(need);
@@ -969,30 +1033,19 @@ esg_status align_impl(esg_scorer* sc, const uint8_t* d_codes, const uint64_t* d_
     return terr(ESG_ERR_BAD_ARGUMENT, "the alignments need %llu CIGAR words, room for %llu",
                 (unsigned long long)need, (unsigned long long)ops_capacity);
   }
-  if (need) {
+  if (n_jobs) {
     uint32_t* d_out = nullptr;
-    TCUDA(cudaMemcpyAsync(d_dst, dst.data(), n_jobs * 8, cudaMemcpyHostToDevice, st));
-    // the packed words go where the trace scratch was (it is no longer needed)
-    if (need * 4 <= sizes[9]) {
-      d_out = (uint32_t*)d_trace;
-    } else {
-      TCUDA(cudaMallocFromPoolAsync((void**)&d_out, need * 4, P.pool, st));
-    }
-    const int cb = (int)std::min<uint64_t>(4096, (n_jobs + 255) / 256);
-    k7_compact<<<cb, 256, 0, st>>>(d_staging, d_job_at, d_dst, d_res2, n_jobs, d_out);
-    TCUDA(cudaGetLastError());
-    TCUDA(cudaMemcpyAsync(ops, d_out, need * 4, cudaMemcpyDeviceToHost, st));
-    TCUDA(cudaStreamSynchronize(st));
-    if ((void*)d_out != (void*)d_trace) cudaFreeAsync(d_out, st);
-  }
-  for (uint32_t k = 0; k < n_jobs; ++k) {
-    out[k].score = res[k].x;
-    out[k].query_start = (uint32_t)res[k].y;
-    out[k].query_end = (uint32_t)res[k].z;
-    out[k].ref_start = (uint32_t)res[k].w;
-    out[k].ref_end = (uint32_t)res2[k].x;
-    out[k].n_ops = (uint32_t)res2[k].y;
-    out[k].ops_offset = dst[k];
+    if (need) TCUDA(cudaMallocFromPoolAsync((void**)&d_out, need * 4, P.pool, st));
+    k7_pack<<<pack_blocks, kPackThreads, 0, st>>>(d_res, d_res2, n_jobs, d_sums, d_staging,
+                                                  d_job_at, d_rec, d_out);
+    cudaError_t e = cudaGetLastError();
+    if (e == cudaSuccess)
+      e = cudaMemcpyAsync(out, d_rec, n_jobs * sizeof(esg_alignment), cudaMemcpyDeviceToHost, st);
+    if (e == cudaSuccess && need)
+      e = cudaMemcpyAsync(ops, d_out, need * 4, cudaMemcpyDeviceToHost, st);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+    if (d_out) cudaFreeAsync(d_out, st);
+    TCUDA(e);
   }
   cudaFreeAsync(mem, st);
   esg_internal_set_error(ESG_OK, "");
@@ -1040,27 +1093,37 @@ esg_status esg_align_reads(esg_scorer* sc, const uint8_t* codes, const uint64_t*
   if (n_reads && (!off || !len)) return terr(ESG_ERR_BAD_ARGUMENT, "off/len must not be NULL");
   esg_internal_panel P{};
   esg_internal_panel_of(sc, &P);
-  // the reads, packed, to the device (no scoring)
+  // the reads to the device (no scoring): packed first, unless they already
+  // lie one after the other
   std::vector<uint64_t> poff(std::max<uint32_t>(n_reads, 1), 0);
   uint64_t total = 0;
+  bool together = true;
   for (uint32_t k = 0; k < n_reads; ++k) {
     poff[k] = total;
+    together = together && off[k] == off[0] + total;
     total += len[k];
   }
   if (total && !codes) return terr(ESG_ERR_BAD_ARGUMENT, "codes must not be NULL");
-  std::vector<uint8_t> pc(std::max<uint64_t>(total, 1));
-  for (uint32_t k = 0; k < n_reads; ++k)
-    if (len[k]) memcpy(pc.data() + poff[k], codes + off[k], len[k]);
+  std::vector<uint8_t> pc;
+  const uint8_t* src = nullptr;
+  if (total && together) {
+    src = codes + off[0];
+  } else if (total) {
+    pc.resize(total);
+    for (uint32_t k = 0; k < n_reads; ++k)
+      if (len[k]) memcpy(pc.data() + poff[k], codes + off[k], len[k]);
+    src = pc.data();
+  }
   cudaSetDevice(P.device);
   cudaStream_t st = P.stream;
-  const size_t b0 = align256(pc.size()), b1 = align256(poff.size() * 8),
+  const size_t b0 = align256(std::max<uint64_t>(total, 1)), b1 = align256(poff.size() * 8),
                b2 = align256(std::max<uint32_t>(n_reads, 1) * 4);
   void* mem = nullptr;
   TCUDA(cudaMallocFromPoolAsync(&mem, b0 + b1 + b2, P.pool, st));
   uint8_t* d_codes = (uint8_t*)mem;
   uint64_t* d_off = (uint64_t*)((char*)mem + b0);
   uint32_t* d_len = (uint32_t*)((char*)mem + b0 + b1);
-  TCUDA(cudaMemcpyAsync(d_codes, pc.data(), pc.size(), cudaMemcpyHostToDevice, st));
+  if (total) TCUDA(cudaMemcpyAsync(d_codes, src, total, cudaMemcpyHostToDevice, st));
   TCUDA(cudaMemcpyAsync(d_off, poff.data(), poff.size() * 8, cudaMemcpyHostToDevice, st));
   if (n_reads) TCUDA(cudaMemcpyAsync(d_len, len, n_reads * 4, cudaMemcpyHostToDevice, st));
   const esg_status s = align_impl(sc, d_codes, d_off, d_len, n_reads, len, jobs, n_jobs, out,

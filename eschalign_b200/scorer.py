@@ -568,10 +568,7 @@ class GpuScorer:
         here): coordinates and CIGAR of each, as scalar::align gives them."""
         codes, off, lens = self._inputs(reads)
         jobs = _jobs_array(jobs)
-        ref_len = self._panel_arrays[2]
-        bound = int(lens[jobs[:, 0]].sum(dtype=np.uint64) + ref_len[jobs[:, 1]].sum(dtype=np.uint64)) \
-            if jobs.shape[0] and (jobs[:, 0] < lens.size).all() and (jobs[:, 1] < ref_len.size).all() \
-            else 0
+        bound = _words_bound(jobs, lens, self._panel_arrays[2])
         return _align_call(self._lib, self._lib.esg_align_reads,
                            (self._h, _ptr(codes, C.c_uint8), _ptr(off, C.c_uint64),
                             _ptr(lens, C.c_uint32), lens.size), jobs, bound)
@@ -581,12 +578,7 @@ class GpuScorer:
         (finish it with keep=True)."""
         jobs = _jobs_array(jobs)
         lens = getattr(batch, "lens", None)
-        ref_len = self._panel_arrays[2]
-        bound = 0
-        if lens is not None and jobs.shape[0] and (jobs[:, 0] < lens.size).all() and \
-                (jobs[:, 1] < ref_len.size).all():
-            bound = int(lens[jobs[:, 0]].sum(dtype=np.uint64) +
-                        ref_len[jobs[:, 1]].sum(dtype=np.uint64))
+        bound = 0 if lens is None else _words_bound(jobs, lens, self._panel_arrays[2])
         return _align_call(self._lib, self._lib.esg_align_batch, (self._h, batch._h), jobs, bound)
 
     # -- mapping (mapper.rs:400-552)
@@ -880,12 +872,26 @@ class Mappings:
                 "hits": hits}
 
 
+def _words_bound(jobs, lens, ref_len) -> int:
+    """An upper bound on the jobs' CIGAR words (runs <= read + reference
+    length per job): from the longest of each while that is small -- the room
+    is only touched where words are written -- else job by job."""
+    if not jobs.shape[0] or not lens.size:
+        return 0
+    cheap = jobs.shape[0] * (int(lens.max()) + int(ref_len.max()))
+    if cheap <= 1 << 28:
+        return cheap
+    if not ((jobs[:, 0] < lens.size).all() and (jobs[:, 1] < ref_len.size).all()):
+        return 0
+    return int(lens[jobs[:, 0]].sum(dtype=np.uint64) + ref_len[jobs[:, 1]].sum(dtype=np.uint64))
+
+
 def _align_call(lib, fn, args_head, jobs, bound=0):
     """One call with room for `bound` words (an upper bound when known:
     runs <= read + reference length per job), a second if it was short."""
     jobs = _jobs_array(jobs)
     n = jobs.shape[0]
-    rec = np.zeros(max(n, 1), dtype=ALIGN_DTYPE)
+    rec = np.empty(max(n, 1), dtype=ALIGN_DTYPE)  # every record is written
     need = C.c_uint64()
     cap = int(bound)
     ops = np.empty(max(cap, 1), dtype=np.uint32)  # only the words written are touched
