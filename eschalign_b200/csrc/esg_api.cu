@@ -200,8 +200,11 @@ struct esg_scorer {
   // batched kernel (0: none; set by the autotuner where the batched kernel
   // would flag most of them)
   uint32_t int32_from = 0;
-  // panel chunking aims for this many tasks per resident warp
-  uint32_t chunk_target = 8;
+  // panel chunking aims for this many tasks per resident warp: the last wave is
+  // idle half the time, and merging the chunks' states costs little (at 8, 16,
+  // 32: 25 000 pairs 37.2, 36.1, 35.9 ms; 50 000 reads 39.0, 38.9, 38.5; 300
+  // reads x 3001 references 107.7, 105.7, 104.3)
+  uint32_t chunk_target = 32;
   uint32_t max_chunks = kMaxChunks;  // panel chunks per tile at most (1: never chunk)
   cudaStream_t aux = nullptr;          // second stream: the long-query kernel
   // batches' device memory: a pool of this scorer's own that keeps what
@@ -1050,14 +1053,14 @@ static esg_status autotune_impl(esg_scorer* sc, const std::vector<uint32_t>& his
     cudaEventDestroy(e1);
     return st;
   }
-  // 16-row stripes up to the last length where they are as fast within 2 %
-  // (timing noise), counting from the shortest; 32-row stripes from the
-  // first length they win by more.  The int32 lanes from the length where
+  // 16-row stripes up to the last length where they are the faster, counting
+  // from the shortest; longer stripes (28 and 32 rows) from the first length
+  // where they are.  The int32 lanes from the length where
   // they win at it and every longer length (a scheme whose long queries
   // mostly flag, to be scored twice by the batched kernel), else never.
   uint32_t split = 0;
   for (uint32_t li = 0; li < rep.n_lengths; ++li) {
-    if (rep.ms_rows16[li] <= 1.02f * rep.ms_rows32[li])
+    if (rep.ms_rows16[li] < rep.ms_rows32[li])
       split = rep.lengths[li];
     else
       break;
@@ -1071,9 +1074,7 @@ static esg_status autotune_impl(esg_scorer* sc, const std::vector<uint32_t>& his
       break;
   }
   // 1b. with a sample of the workload's read lengths: every candidate split
-  //     timed on one batch drawn from that histogram, the fastest kept (of
-  //     equal times, within 1 %, the larger split: 16-row tiles carry less
-  //     skew per pair)
+  //     timed on one batch drawn from that histogram, the fastest kept
   if (!hist.empty()) {
     uint64_t bases = 0;
     for (uint32_t v : hist) bases += v;
@@ -1093,8 +1094,8 @@ static esg_status autotune_impl(esg_scorer* sc, const std::vector<uint32_t>& his
       rep.splits[rep.n_splits] = cand;
       rep.ms_splits[rep.n_splits] = ms;
       ++rep.n_splits;
-      if (rep.n_splits == 1 || ms <= 1.01f * best) {
-        if (rep.n_splits == 1 || ms < best) best = ms;
+      if (rep.n_splits == 1 || ms < best) {
+        best = ms;
         split = cand;
       }
     }
@@ -1135,10 +1136,10 @@ static esg_status autotune_impl(esg_scorer* sc, const std::vector<uint32_t>& his
   }
   sc->split_len = split;
   // 3. panel chunking: a batch of about one read per resident warp (too few
-  //    tiles to fill the GPU), chunked to aim for 1-16 tasks per resident warp
+  //    tiles to fill the GPU), chunked to aim for 1-32 tasks per resident warp
   if (st == ESG_OK) {
     calib_reads(sc, 112, (uint32_t)std::max(64, sc->k2[kRows16][0].blocks * kK2Warps), x, c);
-    static const uint32_t kTargets[] = {1, 2, 4, 8, 16};
+    static const uint32_t kTargets[] = {1, 2, 4, 8, 16, 32};
     float best = 0;
     uint32_t pick = keep_target;
     for (uint32_t t : kTargets) {
