@@ -1334,6 +1334,9 @@ static esg_status prepare_impl(esg_scorer* sc, const uint8_t* const* ptrs, const
   b->host_list = n_k3;
   b->redo_cap = redo_cap;
   const bool local = sc->mode == ESG_MODE_LOCAL;
+  // (a mismatch cheaper to write as a gap: only the checked lanes' records are
+  // built for it, see pair_pass)
+  sg_check = sg_check || sc->scoring.mismatch < sc->scoring.gap_open;
   for (int k = 0; k < kShapes; ++k) b->second[k] = local ? half[k] : sg_check;
   auto& qlong = qs[kLongQuery];
   std::stable_sort(qlong.begin(), qlong.end(),

@@ -79,8 +79,8 @@ constexpr uint32_t kHalfOne = 0x3c003c00u;  // 1.0 in both halves
 // 1.4 register moves a cell pair (of 7.9 instructions) on the rotated state;
 // unrolled past about 16 KB of code it outruns the instruction cache.  Swept
 // 1-8 on B200, 150 000 C2 reads on one shape: local f16, 32 rows 133 / 121 /
-// 125 / 122 ms at 1 / 2 / 3 / 4; semi-global, 32 rows 129 / 120 / 126 at 2 /
-// 3 / 4; reading the panel through L2, semi-global 205 at 3, 197 at 6; int16
+// 125 / 122 ms at 1 / 2 / 3 / 4; semi-global, 28 + 32 rows 115 / 114 / 115 at 2 /
+// 3 / 4; reading the panel through L2, semi-global 183 at 3, 181 at 5; int16
 // local 28 + 32 rows 138 / 128 / 130 at 1 / 2 / 3; long queries 53.5 / 63 /
 // 80 at 2 / 4 / 6 (two stripe heights share the cache).
 template <int R, bool kSmem, bool kLong>
@@ -88,7 +88,7 @@ __host__ __device__ constexpr int steady_unroll(bool local, int lanes) {
   if (kLong) return 2;
   if (R == 8) return 4;
   if (lanes == kLanesHalf) return R == 16 ? 3 : kSmem ? 2 : 4;
-  if (!local) return R == 16 || kSmem ? 3 : 6;
+  if (!local) return R == 16 || kSmem ? 3 : 5;
   return R == 16 ? 8 : kSmem ? 2 : 4;
 }
 
@@ -223,7 +223,7 @@ struct K2Params {
   uint32_t tab_a[6];
   uint32_t tab_b[6];
   uint32_t rec2;         // kLanesHalf: added to a table's score to give s (see pair_pass)
-  int32_t borrow;        // semi-global: some s - o is negative
+  int32_t borrow;        // kLanesChecked: some s - o is negative
   uint32_t e2;           // e in both halves
   int32_t o, e;
   int32_t bias;          // value bias of the int16 lanes
@@ -314,19 +314,21 @@ __device__ __forceinline__ bool stage_panel(void* smem, const void* gsrc, uint32
 //     record is written a column ahead), so that nothing old outlives the
 //     update and the registers need no rotation.  The best is taken over d:
 //     E and F never exceed an earlier H.
-//   kLanesInt, semi-global  Halves hold value + B (B = -16384) in int16;
-//     g[r] = G = H + o + B of the row at the previous column.
+//   kLanesInt, semi-global  Halves hold value + B (B = -16384) in int16.
 //     d = G_diag + (s - o) and G = H + o are 32-bit IMADs, exact in both
 //     halves: the low half's sums stay negative (static bound, or watched, see
 //     kLanesChecked), so a negative addend's carry out is the rule, cancelled
-//     by o * 65537 or by a record word built with one less above it
-//     (P.borrow), and the high half's carry is discarded.  Padding columns
-//     (garbage that may wrap) are only ever in the high half.  3 ALU.
+//     by o * 65537 (and, where some s - o is negative, by a record word built
+//     with one less above it: kLanesChecked alone spends the instructions on
+//     that), and the high half's carry is discarded.  Padding columns (garbage
+//     that may wrap) are only ever in the high half.  3 ALU.  g[r] is d of the
+//     row's next column in the unchecked loop, as above, and G of its last one
+//     in the checked one, which takes the columns' ends from it.
 //   kLanesInt, local  B = 2048; d takes the ALU (max(G_diag + (s - o), E)) as
 //     nothing else gives the floor.  4.5 ALU.  For scores past 2047.
 //
 // C2 local, 150 000 reads: 115.8 ms; with 4.5 ALU on 16-row stripes (the best
-// of before) 137.5.  Semi-global 115.7 against 130.7 (5 ALU, 32 rows).
+// of before) 137.5.  Semi-global 107.9 against 130.7 (5 ALU, 32 rows).
 //
 // Score records: at each column the lane writes the column's score word for
 // each read code (PRMT of that code's tables by the column's selector, which
@@ -351,7 +353,7 @@ __device__ __forceinline__ bool stage_panel(void* smem, const void* gsrc, uint32
 // maximum (G, the short half's taken at its own end) in `v`, and the
 // semi-global maximum of the last row over the lane's columns (H + B) in `lr`.
 struct PassConst {
-  uint32_t g0, neg2, e2, o32, one, bias2;
+  uint32_t g0, f0, neg2, e2, o32, one, bias2;
 };
 
 // A column's 16-bit PRMT selector: an explicit shared-memory load when the
@@ -393,10 +395,10 @@ __device__ __forceinline__ void pair_pass(const K2Params& P, uint32_t scr, bool 
 #pragma unroll
   for (int r = 0; r < R; ++r) {
     g[r] = K.g0;
-    ev[r] = K.neg2;
+    ev[r] = K.f0;
   }
   uint32_t gdc = K.g0;  // G of the row above, previous column
-  uint32_t gbot = K.g0, fbot = K.neg2;
+  uint32_t gbot = K.g0, fbot = K.f0;
   // local: max H + B over this lane's cells; checked semi-global: the same
   // without the floor (the short half's taken at its own end)
   uint32_t best = kLocal ? K.bias2 : K.neg2, s_best = K.neg2;
@@ -414,7 +416,7 @@ __device__ __forceinline__ void pair_pass(const K2Params& P, uint32_t scr, bool 
     auto word = [&](int c) {
       uint32_t w = prmt(P.tab_a[c], P.tab_b[c], sel);
       if constexpr (kHalf) w = add_f16x2(w, P.rec2);
-      if constexpr (!kLocal)
+      if constexpr (kCheck)
         if (P.borrow) w -= (w << 1) & 0x10000u;
       st_shared_u32(scr + c * kScrStride, w);
     };
@@ -445,7 +447,7 @@ __device__ __forceinline__ void pair_pass(const K2Params& P, uint32_t scr, bool 
     }
     // columns of a lane come in order: with kPre the next one's selector is
     // loaded a column ahead
-    constexpr int kAhead = kHalf ? 1 : 0;
+    constexpr int kAhead = kHalf || (!kLocal && !kSnap) ? 1 : 0;
     uint32_t sel;
     if constexpr (kPre) {
       sel = seln;
@@ -454,61 +456,76 @@ __device__ __forceinline__ void pair_pass(const K2Params& P, uint32_t scr, bool 
       sel = load_sel<kSmem>(sp, j + kAhead);
     }
     record(sel);
-    if constexpr (kHalf) {
-      uint32_t f = ft, up = gt, prev = 0;
+    if constexpr (kHalf || (!kLocal && !kSnap)) {
+      // g[r]: the row's diagonal term at this column, then at the next
+      uint32_t f = ft, up = gt, prev = 0, h = 0;
 #pragma unroll
       for (int r = 0; r < R; ++r) {
         const uint32_t d = g[r];
-        const uint32_t h = __vimax3_s16x2(d, ev[r], f);
-        if (r & 1)
-          best = __vimax3_s16x2(best, prev, d);
-        else
-          prev = d;
-        g[r] = add_relu_f16x2(up, ld_shared_u32(ta[r]));
-        const uint32_t gr = add_relu_f16x2(h, K.o32);
+        h = __vimax3_s16x2(d, ev[r], f);
+        if constexpr (kLocal || kCheck) {
+          const uint32_t x = kLocal ? d : h;
+          if (r & 1)
+            best = __vimax3_s16x2(best, prev, x);
+          else
+            prev = x;
+        }
+        const uint32_t sc = ld_shared_u32(ta[r]);
+        g[r] = kHalf ? add_relu_f16x2(up, sc) : mad_lo(up, K.one, sc);
+        const uint32_t gr = kHalf ? add_relu_f16x2(h, K.o32) : mad_lo(h, K.one, K.o32);
         ev[r] = __viaddmax_s16x2(ev[r], K.e2, gr);
         f = __viaddmax_s16x2(f, K.e2, gr);
-        up = h;
+        up = kHalf ? h : gr;
       }
       gbot = up;
       fbot = f;
+      if constexpr (!kLocal) lastrow = max16x2(lastrow, h);
       if constexpr (kLong) {
         if (to_buf && lane == 31) buf[j] = make_uint2(gbot, fbot);
       }
       return;
     }
-    uint32_t gup = gt, f = ft, h15 = 0, hprev = 0, gd = gdc;
+    uint32_t f = ft, h15 = 0, hprev = 0, gd = gdc;
     gdc = gt;
-    // semi-global: a row's diagonal term is taken before the row above
-    // overwrites the G it reads, which lets every g[r] stay in its register
-    auto diag = [&](int r) {
-      return mad_lo(r ? g[r ? r - 1 : 0] : gd, K.one, ld_shared_u32(ta[r]));
-    };
-    uint32_t dn = kLocal ? 0u : diag(0);
+    if constexpr (kLocal) {
+      uint32_t gup = gt;
 #pragma unroll
-    for (int r = 0; r < R; ++r) {
-      const uint32_t d = dn;
-      if constexpr (!kLocal)
-        if (r + 1 < R) dn = diag(r + 1 < R ? r + 1 : r);
-      ev[r] = __viaddmax_s16x2(ev[r], K.e2, g[r]);
-      f = __viaddmax_s16x2(f, K.e2, gup);
-      uint32_t h;
-      if constexpr (kLocal) {
+      for (int r = 0; r < R; ++r) {
+        ev[r] = __viaddmax_s16x2(ev[r], K.e2, g[r]);
+        f = __viaddmax_s16x2(f, K.e2, gup);
         const uint32_t h1 = __viaddmax_s16x2(gd, ld_shared_u32(ta[r]), ev[r]);
         gd = g[r];
-        h = __vimax3_s16x2(h1, f, K.bias2);
-      } else {
-        h = __vimax3_s16x2(d, ev[r], f);
-      }
-      if constexpr (kLocal || kCheck) {
+        const uint32_t h = __vimax3_s16x2(h1, f, K.bias2);
         if (r & 1)
           best = __vimax3_s16x2(best, hprev, h);
         else
           hprev = h;
+        g[r] = mad_lo(h, K.one, K.o32);
+        gup = g[r];
       }
-      g[r] = mad_lo(h, K.one, K.o32);
-      gup = g[r];
-      if (r == R - 1) h15 = h;
+    } else {
+      // (a row's diagonal term is taken before the row above overwrites the G
+      // it reads)
+      auto diag = [&](int r) {
+        return mad_lo(r ? g[r ? r - 1 : 0] : gd, K.one, ld_shared_u32(ta[r]));
+      };
+      uint32_t dn = diag(0);
+#pragma unroll
+      for (int r = 0; r < R; ++r) {
+        const uint32_t d = dn;
+        if (r + 1 < R) dn = diag(r + 1 < R ? r + 1 : r);
+        const uint32_t h = __vimax3_s16x2(d, ev[r], f);
+        if constexpr (kCheck) {
+          if (r & 1)
+            best = __vimax3_s16x2(best, hprev, h);
+          else
+            hprev = h;
+        }
+        g[r] = mad_lo(h, K.one, K.o32);
+        ev[r] = __viaddmax_s16x2(ev[r], K.e2, g[r]);
+        f = __viaddmax_s16x2(f, K.e2, g[r]);
+        if (r == R - 1) h15 = h;
+      }
     }
     gbot = g[R - 1];
     fbot = f;
@@ -545,7 +562,7 @@ __device__ __forceinline__ void pair_pass(const K2Params& P, uint32_t scr, bool 
     ft = __shfl_up_sync(kFull, fbot, 1);
     if (first) {
       gt = K.g0;
-      ft = K.neg2;
+      ft = K.f0;
     }
   };
 
@@ -566,15 +583,29 @@ __device__ __forceinline__ void pair_pass(const K2Params& P, uint32_t scr, bool 
       uint32_t gt, ft;
       top(gt, ft);
       const int j = t - skew;
-      if ((unsigned)j < (unsigned)mlim) column(IntConst<0>{}, j, gt, ft);
+      if ((unsigned)j < (unsigned)mlim) column(IntConst<kLocal ? 0 : 1>{}, j, gt, ft);
     }
     const int sk = active_lane ? skew : 0;
+    if constexpr (!kLocal) {
+      // from G of the last column to the diagonal terms of the next
+      record(load_sel<kSmem>(sp, t - sk));
+#pragma unroll
+      for (int r = R - 1; r >= 0; --r)
+        g[r] = mad_lo(r ? g[r ? r - 1 : 0] : gdc, K.one, ld_shared_u32(ta[r]));
+    }
     constexpr int kUnroll = steady_unroll<R, kSmem, kLong>(kLocal, kLanes);
 #pragma unroll kUnroll
     for (; t < full; ++t) {
       uint32_t gt, ft;
       top(gt, ft);
       column(IntConst<0>{}, t - sk, gt, ft);
+    }
+    if constexpr (!kLocal) {
+      // and back: the next column's record is in place
+      gdc = g[0] - ld_shared_u32(ta[0]);
+#pragma unroll
+      for (int r = 0; r + 1 < R; ++r) g[r] = g[r + 1 < R ? r + 1 : r] - ld_shared_u32(ta[r + 1 < R ? r + 1 : r]);
+      g[R - 1] = gbot;
     }
   }
 #pragma unroll 1
@@ -690,8 +721,8 @@ __device__ __forceinline__ void flush_query(const K2Params& P, uint32_t qid, uin
 // scored in ceil(S / 32) passes per pair chained through a per-warp column
 // buffer in global memory, the last one on 16-row stripes when that is enough
 // (half the lanes' rows would be idle: 600 reads of 1100-5000 nt against 48
-// references, with the unrolled loop, 74.6 -> 53.5 ms semi-global, 75.0 ->
-// 57.3 local).  Instantiations of their own keep the register allocation of
+// references, with the unrolled loop, 74.6 -> 47.1 ms semi-global, 75.0 ->
+// 55.2 local).  Instantiations of their own keep the register allocation of
 // the short-read path free of the long path's state.
 // Stripes are aligned so the read's last row is the last row of its last
 // stripe; the rows before the read's first row score 0 against every real
@@ -733,6 +764,10 @@ __global__ void __launch_bounds__(kK2Threads, R > 16 ? ESG_K2_R32_BLOCKS : ESG_K
   // a zero border cell's G (kLanesHalf: its H) and its E and F
   K.g0 = kHalf ? 0u : pack16x2(bias + P.o, bias + P.o);
   K.neg2 = kHalf ? 0u : pack16x2(kNeg16, kNeg16);
+  // E of column 1 and F of row 1: semi-global, opened at the zero border;
+  // int16 local takes them a cell later (its E and F are the last column's and
+  // the row above's)
+  K.f0 = kHalf || kLocal ? K.neg2 : K.g0;
   K.bias2 = pack16x2(bias, bias);  // H = 0 (the local floor)
   // + o in both halves: one 32-bit add, or one f16x2 add
   K.o32 = kHalf ? half_pair(P.o) : (uint32_t)(P.o * 65537);
