@@ -1150,8 +1150,9 @@ static esg_status autotune_impl(esg_scorer* sc, const std::vector<uint32_t>& his
       rep.chunk_targets[rep.n_chunk_targets] = t;
       rep.ms_chunks[rep.n_chunk_targets] = ms;
       ++rep.n_chunk_targets;
-      if (rep.n_chunk_targets == 1 || ms < best) {
-        best = ms;
+      // (of equal times, within 1 %, the finer chunks: larger batches gain)
+      if (rep.n_chunk_targets == 1 || ms < 1.01f * best) {
+        best = rep.n_chunk_targets == 1 ? ms : std::min(best, ms);
         pick = t;
       }
     }

@@ -79,3 +79,38 @@ def test_scorers_over_panels_of_different_sizes(oracle):
         assert (h.score_batch(reads, full_rows=True).rows ==
                 oracle.score_matrix(reads, small, (2, -1, -10, -1), True)).all()
     assert (rows == oracle.score_matrix(reads, big, (2, -1, -10, -1), True)).all()
+
+
+@pytest.mark.parametrize("mode", [Mode.LOCAL, Mode.SEMIGLOBAL])
+@pytest.mark.parametrize("cap", [1, 8, 32])
+def test_small_batches_without_a_split(oracle, mode, cap):
+    """A scorer left to itself puts a few reads on 8- or 16-row stripes, a
+    panel chunk per reference pair, and merges the chunks straight into the
+    results: one to forty reads (empty ones, ones past those stripes among
+    them) against one to 90 references, a third of them the same, so that tie
+    sets span many chunks and outrun the list."""
+    rng = np.random.default_rng(cap)
+    same = rng.integers(0, 4, 60).astype(np.uint8)
+    panel = [same if k % 3 == 0 else rng.integers(0, 4, int(rng.integers(20, 140))).astype(np.uint8)
+             for k in range(90)]
+    sc = (2, -1, -10, -1)
+    local = mode == Mode.LOCAL
+    for n_refs in (1, 2, 90):
+        refs = panel[:n_refs]
+        with GpuScorer(refs, Scoring(*sc), mode, tie_capacity=cap) as g:
+            for lens in ([60], [0, 8, 9], [255, 256, 257, 513, 0], SHORT + SHORT[::-1]):
+                reads = _reads(rng, refs, lens)
+                want, ties, _ = oracle.scalar_map_batch(reads, refs, sc, local, True, cap=cap)
+                got = g.score_batch(reads, both_strands=True)
+                for f in ("best", "suboptimal", "n_tied"):
+                    assert (got.results[f] == want[f]).all(), (n_refs, lens, f)
+                for k in range(len(reads)):
+                    m = min(int(want["n_tied"][k]), cap)
+                    assert list(got.ties[k, :m]) == list(ties[k][:m]), (n_refs, lens, k)
+                    assert (got.ties[k, m:] == 0xFFFFFFFF).all()
+                rows = g.score_batch(reads, both_strands=True, full_rows=True).rows
+                rc = [oracle.revcomp(r) for r in reads]
+                assert (rows == oracle.score_matrix(reads + rc, refs, sc, local)).all()
+                one = g.score_batch(reads)
+                fwd, _, _ = oracle.scalar_map_batch(reads, refs, sc, local, False, cap=cap)
+                assert (one.results["best"] == fwd["best"]).all()
