@@ -74,11 +74,12 @@ COMBOS = [((2, -1, -10, -1), "local"), ((2, -1, -10, -1), "semiglobal"),
 OPS_PER_CELL = {"local": 12, "semiglobal": 11}
 C4_SCORING = (2, -1, -10, -1)
 C3_SCORING = (2, -1, -10, -1)
-# DRAM bytes per DP cell of the batched kernel: 8.29 MB read, 0 written, over
-# the 2.678e11 cells of the 16-row launch in the ncu capture of a 60 000-read
-# C2 case (profiles/k2_batched_c2.md); the traffic is the reads' codes and
-# the plan, which grow with the reads, so it scales by cells to a full launch.
-K2_DRAM_BYTES_PER_CELL = 8.288256e6 / 2.67805237160e11
+# DRAM bytes per DP cell of the batched kernel: 36.95 MB read, 5.11 MB
+# written, over the 7.308e11 cells of the 28- and 32-row launches in the ncu
+# capture of a 150 000-read C2 case (profiles/k2_batched_c2.md); the traffic is
+# the reads' codes, the plan and the results, which grow with the reads, so it
+# scales by cells to a full launch.
+K2_DRAM_BYTES_PER_CELL = (36.953344e6 + 5.105664e6) / 7.30839703376e11
 
 
 def env_int(name, default):

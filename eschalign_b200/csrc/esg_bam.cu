@@ -1774,7 +1774,7 @@ esg_status esg_bam_writer_blocks(const esg_bam_writer* w, uint64_t* blocks,
   return ESG_OK;
 }
 
-// The device deflate's steps run on the host, lane by lane: one block of at
+// The device deflate's steps run on the host, stripe by stripe: one block of at
 // most 0xff00 bytes into `out` (65536 bytes, 4-byte aligned).  Returns the
 // DEFLATE length, 0xffffffff for "store it", 0 on a bad argument.  A check
 // of the steps for tests; the writer never calls it.

@@ -723,7 +723,7 @@ esg_status esg_bam_writer_use_device(esg_bam_writer* writer, int32_t device);
 /* Blocks written by the device so far, and how many of them stored. */
 esg_status esg_bam_writer_blocks(const esg_bam_writer* writer, uint64_t* blocks,
                                  uint64_t* stored);
-/* The device compressor's steps run on the host, lane by lane, on one block
+/* The device compressor's steps run on the host, stripe by stripe, on one block
  * (1 <= n <= 0xff00 bytes) into `out` (65536 bytes, 4-byte aligned): the
  * length of the raw DEFLATE stream, 0xffffffff when the block is to be
  * stored, 0 on a bad argument.  For checking the steps without a device;
