@@ -456,13 +456,14 @@ __device__ __forceinline__ void tag_tile(const K7TagParams& P, const int4* tab, 
     tag_sts(my + 2 * kStride, (uint32_t)tw.z);
     tag_sts(my + 3 * kStride, (uint32_t)tw.w);
   };
-  // d of the row's next column
+  // d of the row's next column, and E of the first one: opened at the border,
+  // as F of a first row is (local, where an open from 0 is under the floor: the floor)
   int g[R], ev[R];
   record(valid ? rp[0] : 0);
 #pragma unroll
   for (int r = 0; r < R; ++r) {
     g[r] = add(kZero, (int)tag_lds(addr[r]));
-    ev[r] = kLocal ? 0 : kTagNeg;
+    ev[r] = kLocal ? 0 : add(kZero, cE);
   }
   int x1 = rp[min(1, last)];
   int hbot = kZero, fbot = add(kZero, cF);

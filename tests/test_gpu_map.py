@@ -312,3 +312,23 @@ def test_map_two_scorers_on_two_threads():
     finally:
         for g in gs:
             g.close()
+
+
+@pytest.mark.parametrize("mode", [Mode.LOCAL, Mode.SEMIGLOBAL])
+@pytest.mark.parametrize("scoring", [(1, -4, -6, -1), (2, -3, -2, -1), (2, -3, -1, -5),
+                                     (100, -100, -200, -30)])
+def test_map_reads_over_a_references_ends(oracle, mode, scoring):
+    """Schemes whose gap from the border beats a mismatch: the hits' scores
+    and CIGARs (a leading deletion among them) equal the oracle's."""
+    rng = Rng(0x5EED_0B0D)
+    panel = [random_seq(rng, n, 0.0) for n in (23, 40, 70, 110)]
+    reads = []
+    for k, ref in enumerate(panel * 6):
+        n = 1 + k % 6
+        body = bytes(b"TGCA"[b"ACGT".index(c)] for c in ref[:n]) + ref[n:]
+        reads.append(random_seq(rng, 1 + 3 * k % 41, 0.0) + body)
+        reads.append(ref[:-n] + body[:n] + random_seq(rng, 1 + 3 * k % 41, 0.0))
+    got, want = run(oracle, panel, reads, scoring, mode, both_strands=True)
+    for k in range(len(reads)):
+        m = got.mapping(k)
+        assert all(h["score"] == m["best_score"] for h in m["hits"])

@@ -181,3 +181,53 @@ def test_trace_tagged_values_at_their_edges(oracle, mode):
         with GpuScorer(panel, Scoring(*scoring), mode) as g:
             check(oracle, g, reads, panel, jobs, scoring, mode == Mode.LOCAL,
                   f"tags {mode.label} {scoring}")
+
+
+# a mismatch below the gap open, or below the extension: a gap from the border
+# beats a mismatch at the first or last bases
+BORDER_GAPS = [(1, -4, -6, -1), (5, -4, -8, -1), (2, -3, -2, -1), (2, -3, -1, -5), (1, -4, -2, -1),
+               (2, -8, -4, -2), (100, -100, -200, -30)]
+
+
+def overhanging_read(rng, ref, lead, changed):
+    """`lead` bases before the reference, with its first `changed` ones changed."""
+    body = ref.copy()
+    body[:changed] = np.where(body[:changed] > 3, 0, 3 - body[:changed])
+    return np.concatenate([rng.integers(0, 4, lead).astype(np.uint8), body])
+
+
+@pytest.mark.parametrize("mode", [Mode.LOCAL, Mode.SEMIGLOBAL])
+@pytest.mark.parametrize("scoring", BORDER_GAPS)
+def test_trace_gaps_from_the_border(oracle, mode, scoring):
+    """A deletion of a reference's first bases is opened at the zero border,
+    in the first column of every row of a stripe, as an insertion is in the
+    first row: reads that hang over a reference's start or, mirrored, its end,
+    of lengths on both sides of a stripe of 28 and 32 rows."""
+    rng = np.random.default_rng(0xB0D)
+    panel = [rng.integers(0, 5 if m == 90 else 4, m).astype(np.uint8)
+             for m in (7, 20, 27, 28, 33, 60, 90, 140)]
+    reads = []
+    for k, lead in enumerate((1, 2, 5, 8, 17, 40)):
+        for j, ref in enumerate(panel):
+            reads.append(overhanging_read(rng, ref, lead, 1 + (j + k) % 6))
+            reads.append(overhanging_read(rng, ref[::-1], lead, 1 + (j + k) % 6)[::-1].copy())
+    jobs = [(i, r, v) for i in range(len(reads)) for r in range(len(panel)) for v in (0, 1)
+            if r == i // 2 % len(panel) or (i + r) % 5 == 0]
+    with GpuScorer(panel, Scoring(*scoring), mode) as g:
+        got = check(oracle, g, reads, panel, jobs, scoring, mode == Mode.LOCAL,
+                    f"border {mode.label} {scoring}")
+        rows = g.score_batch(reads, both_strands=True, full_rows=True).rows
+    for k, (rd, ref, rev) in enumerate(jobs):
+        assert int(got.records[k]["score"]) == int(rows[rd + rev * len(reads), ref])
+
+
+def test_trace_leading_deletion_by_hand(oracle):
+    """A deletion of three bases and twenty matches, worked out by hand."""
+    ref, read = encode("GGGACGTTGCAAGCTTACGATCA"), encode("CCCCCACGTTGCAAGCTTACGATCA")
+    for scoring, score in (((1, -4, -6, -1), 12), ((5, -4, -8, -1), 90), ((2, -3, -2, -1), 36),
+                           ((100, -100, -200, -30), 1740)):
+        with GpuScorer([ref], Scoring(*scoring), Mode.SEMIGLOBAL) as g:
+            got = g.align([read], [(0, 0, 0)])
+        rec = got.records[0]
+        assert (int(rec["score"]), got.cigar(0), int(rec["query_start"]), int(rec["query_end"]),
+                int(rec["ref_start"]), int(rec["ref_end"])) == (score, "3D20M", 5, 25, 0, 23)
