@@ -87,6 +87,8 @@ K2Shape shape_of(uint32_t n) {
 
 // Panel chunks per tile at most, unless esg_scorer_set_chunking says less.
 constexpr uint32_t kMaxChunks = 1024;
+// Device memory the panel chunks' states may take (per batch).
+constexpr uint64_t kPartBudget = 1ull << 30;
 
 // A batch's device counters: [1] re-score requests, [2] error bits, [6..7]
 // k3's 64-bit unit counter, one task counter per k2 shape in the others.
@@ -1367,6 +1369,14 @@ static esg_status prepare_impl(esg_scorer* sc, const uint8_t* const* ptrs, const
     if (tiles && tiles < target) nc = (uint32_t)((target + tiles - 1) / tiles);
     nc = std::min<uint32_t>(nc, sc->n_pairs);
     nc = std::min<uint32_t>(nc, sc->max_chunks);
+    // The chunks' states are held for every query, those the tiles do not
+    // hold (empty, or on the int32 lanes) too: at most what full tiles of
+    // them all would be cut into, or 64 a query, inside kPartBudget.  A batch
+    // whose queries are all in tiles is never held back by it; one read among
+    // 20 000 empty ones against 2100 references took 2.0 GB in 1024 chunks.
+    const uint64_t rows = std::max<uint32_t>(b->n_q, 1), row_bytes = 16 + 4ull * sc->cap;
+    nc = (uint32_t)std::min<uint64_t>(nc, std::max<uint64_t>(64, (32 * target + rows - 1) / rows));
+    nc = (uint32_t)std::min<uint64_t>(nc, kPartBudget / (rows * row_bytes));
     b->n_chunks = std::max<uint32_t>(nc, 1);
   }
 

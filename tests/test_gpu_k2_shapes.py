@@ -114,3 +114,41 @@ def test_small_batches_without_a_split(oracle, mode, cap):
                 one = g.score_batch(reads)
                 fwd, _, _ = oracle.scalar_map_batch(reads, refs, sc, local, False, cap=cap)
                 assert (one.results["best"] == fwd["best"]).all()
+
+
+@pytest.mark.parametrize("kernel", ["empty", "int32"])
+def test_chunk_states_of_few_tiled_queries(oracle, kernel):
+    """One read for the batched kernel among 20 000 that are empty (or, past
+    what its lanes hold, on the int32 lanes): the panel is cut into chunks for
+    the one, but the memory of their states, held for every query, stays
+    within 64 chunks a query or 32 queries to each of the device's tasks."""
+    rng = np.random.default_rng(21)
+    same = rng.integers(0, 4, 12).astype(np.uint8)
+    panel = [same if k % 5 == 0 else rng.integers(0, 4, int(rng.integers(8, 14))).astype(np.uint8)
+             for k in range(2100)]
+    n, cap, sc = 20_000, 8, (2, -1, -10, -1)
+    reads = [np.zeros(0, np.uint8)] * n
+    mode = Mode.LOCAL
+    if kernel == "int32":
+        # semi-global lanes hold 2 |open| + (min(n, L) - 1) |extend| < 15000:
+        # with this extension reads up to 15 bases of a 16-base reference
+        sc, mode = (2, -1, -10, -1000), Mode.SEMIGLOBAL
+        panel[7] = rng.integers(0, 4, 40).astype(np.uint8)
+        reads = [rng.integers(0, 4, 30).astype(np.uint8) for _ in range(n)]
+    reads[n // 2] = same.copy()
+    with GpuScorer(panel, Scoring(*sc), mode, tie_capacity=cap) as g:
+        tasks = 32 * 4 * g.info()["batched_blocks"]
+        got = g.score_batch(reads, both_strands=True)
+    st = got.stats
+    assert st["queries_batched"] == 2 and st["panel_chunks"] > 1
+    n_q, row = 2 * n, 16 + 4 * cap
+    assert st["panel_chunks"] <= max(64, -(-32 * tasks // n_q))
+    rest = 64 * n_q + (n_q + 2) * row + 4 * len(panel) * (n_q if kernel == "int32" else 1) + (1 << 20)
+    assert st["device_bytes"] <= max(64 * n_q, 32 * tasks + n_q) * row + rest
+    want, ties, _ = oracle.scalar_map_batch(reads[n // 2:n // 2 + 1], panel, sc,
+                                            mode == Mode.LOCAL, True, cap=cap)
+    for f in ("best", "suboptimal", "n_tied"):
+        assert got.results[f][n // 2] == want[f][0], f
+    assert list(got.ties[n // 2, :cap]) == list(ties[0][:cap])
+    if kernel == "empty":
+        assert (np.delete(got.results["flags"], n // 2) & 1).all()
