@@ -85,6 +85,10 @@ K2Shape shape_of(uint32_t n) {
   return (n + 27) / 28 * 28 * 1045 < (n + 31) / 32 * 32 * 1000 ? kRows28 : kRows32;
 }
 
+// Resident CTAs an SM of the long-query kernel: its registers (164-168) allow
+// no more.
+constexpr int kLongBlocks = ESG_K2_R32_BLOCKS;
+
 // Panel chunks per tile at most, unless esg_scorer_set_chunking says less.
 constexpr uint32_t kMaxChunks = 1024;
 // Device memory the panel chunks' states may take (per batch).
@@ -189,7 +193,7 @@ struct esg_scorer {
   // task groups whose queries stay inside them (k2_half).
   struct K2Kernel {
     const void* fn = nullptr;
-    int blocks = 0;      // CTAs launched at most
+    int blocks = 0;      // CTAs launched at most (0: not asked for yet, see k2_ready)
     int occupancy = 0;   // the same, all that fit (the autotuner may lower blocks)
   };
   K2Kernel k2[kShapes][2];
@@ -410,6 +414,26 @@ void set_k2_fn(esg_scorer* sc) {
     sc->k2[kRows8][w].fn = pick_k2<8, false>(local, lanes, smem);
   }
   sc->k3_fn = local ? (const void*)k3_lanes<true> : (const void*)k3_lanes<false>;
+}
+
+// A kernel's shared-memory limit and CTAs, when a batch first takes it: a
+// process's first call to name a kernel loads it, and a first scorer that named
+// all ten of its mode took 17 ms against 15.
+cudaError_t k2_ready(esg_scorer* sc, int shape, bool second) {
+  esg_scorer::K2Kernel& k = sc->k2[shape][second];
+  if (k.blocks) return cudaSuccess;
+  // (the attribute is the process's: every scorer sets the same limit, or
+  // one over a smaller panel would take it from the others)
+  cudaError_t e = cudaFuncSetAttribute(k.fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       (int)kK2SmemLimit);
+  int occ = 0;
+  if (e == cudaSuccess)
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k.fn, kK2Threads, sc->k2_smem);
+  if (e != cudaSuccess) return e;
+  // the long queries' column buffer has room for this many
+  if (shape == kLongQuery) occ = std::min(occ, kLongBlocks);
+  k.blocks = k.occupancy = std::max(1, occ) * sc->sm_count;
+  return cudaSuccess;
 }
 
 // 32-lane tiles of query stripes: best-fit decreasing.  `qs` holds
@@ -758,13 +782,8 @@ esg_status esg_scorer_new(int32_t device, const uint8_t* ref_codes, const uint64
   sc->smem_panel = (size_t)sc->blob_bytes + slots <= kK2SmemLimit;
   set_k2_fn(sc);
   sc->k2_smem = (sc->smem_panel ? sc->blob_bytes : 0) + slots;
-  // (the attribute is the process's: every scorer sets the same limit, or
-  // one over a smaller panel would take it from the others)
-  for (auto& shape : sc->k2)
-    for (auto& k : shape)
-      if ((e = cudaFuncSetAttribute(k.fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    (int)kK2SmemLimit)) != cudaSuccess)
-        return cleanup(cuda_fail(e, "cudaFuncSetAttribute(k2)"));
+  if ((e = k2_ready(sc, kRows16, false)) != cudaSuccess)
+    return cleanup(cuda_fail(e, "cudaFuncSetAttribute(k2)"));
   if ((e = cudaStreamCreateWithFlags(&sc->aux, cudaStreamNonBlocking)) != cudaSuccess ||
       (e = cudaEventCreateWithFlags(&sc->fork, cudaEventDisableTiming)) != cudaSuccess ||
       (e = cudaEventCreateWithFlags(&sc->join, cudaEventDisableTiming)) != cudaSuccess)
@@ -785,20 +804,10 @@ esg_status esg_scorer_new(int32_t device, const uint8_t* ref_codes, const uint64
   if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ3, sc->k3_fn, kK3Threads, 0)) !=
       cudaSuccess)
     return cleanup(cuda_fail(e, "cudaOccupancy"));
-  for (auto& shape : sc->k2)
-    for (auto& k : shape) {
-      int occ = 0;
-      if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k.fn, kK2Threads,
-                                                             sc->k2_smem)) != cudaSuccess)
-        return cleanup(cuda_fail(e, "cudaOccupancy"));
-      k.blocks = k.occupancy = std::max(1, occ) * sc->sm_count;
-    }
-  // the long-query column buffer below is sized for the first kernel's CTAs
-  sc->k2[kLongQuery][1].blocks =
-      std::min(sc->k2[kLongQuery][1].blocks, sc->k2[kLongQuery][0].blocks);
   if (sc->batched_ok && max_len <= 8192) {
     sc->lbuf_cols = max_len;
-    const size_t lb = (size_t)sc->k2[kLongQuery][0].blocks * kK2Warps * max_len * sizeof(uint2);
+    const size_t lb =
+        (size_t)kLongBlocks * sc->sm_count * kK2Warps * max_len * sizeof(uint2);
     if ((e = cudaMalloc(&sc->d_lbuf, lb)) != cudaSuccess)
       return cleanup(cuda_fail(e, "cudaMalloc(long-query buffer)"));
   }
@@ -991,6 +1000,9 @@ static esg_status autotune_impl(esg_scorer* sc, const std::vector<uint32_t>& his
   g_err.clear();
   if (!sc) return fail(ESG_ERR_BAD_ARGUMENT, "NULL scorer");
   esg_tune_report rep{};
+  ESG_CUDA(cudaSetDevice(sc->device));
+  for (int shape : {kRows16, kRows28, kRows32})
+    for (bool second : {false, true}) ESG_CUDA(k2_ready(sc, shape, second));
   rep.chunk_target = sc->chunk_target;
   rep.ctas16 = sc->k2[kRows16][0].blocks / std::max(1, sc->sm_count);
   rep.ctas32 = sc->k2[kRows32][0].blocks / std::max(1, sc->sm_count);
@@ -1000,7 +1012,6 @@ static esg_status autotune_impl(esg_scorer* sc, const std::vector<uint32_t>& his
     if (out) *out = rep;
     return ESG_OK;
   }
-  ESG_CUDA(cudaSetDevice(sc->device));
   static const uint32_t kLens[] = {48, 80, 112, 160, 224, 320, 448};
   const uint32_t n_lens = sizeof(kLens) / sizeof(kLens[0]);
   const uint32_t keep_split = sc->split_len, keep_from = sc->int32_from;
@@ -1870,6 +1881,8 @@ esg_status esg_submit(esg_scorer* sc, esg_batch* b) {
   const size_t np = b->paired ? std::max<uint32_t>(b->n_pairs, 1) : 0;
   const uint32_t nlist = b->host_list + b->redo_cap;
   const size_t nr = b->n_reads ? b->n_reads : 1, nq = b->n_q ? b->n_q : 1;
+  for (int k = 0; k < kShapes; ++k)
+    if (b->n_tiles[k]) ESG_CUDA(k2_ready(sc, k, b->second[k]));
   // device buffers, one stream-ordered allocation
   const size_t total = batch_device_bytes(sc, b);
   ESG_CUDA(cudaMallocFromPoolAsync(&b->d_mem, total, sc->pool, st));
