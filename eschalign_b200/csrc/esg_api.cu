@@ -913,8 +913,8 @@ int32_t esg_batched_takes(const esg_scorer* sc, uint64_t len) {
 esg_status esg_scorer_set_chunking(esg_scorer* sc, uint32_t max_chunks) {
   g_err.clear();
   if (!sc) return fail(ESG_ERR_BAD_ARGUMENT, "NULL scorer");
-  if (max_chunks < 1 || max_chunks > 64)
-    return fail(ESG_ERR_BAD_ARGUMENT, "max_chunks %u outside 1..64", max_chunks);
+  if (max_chunks < 1 || max_chunks > kMaxChunks)
+    return fail(ESG_ERR_BAD_ARGUMENT, "max_chunks %u outside 1..%u", max_chunks, kMaxChunks);
   sc->max_chunks = max_chunks;
   return ESG_OK;
 }

@@ -449,7 +449,8 @@ class GpuScorer:
         _check(self._lib, self._lib.esg_scorer_set_graphs(self._h, int(bool(enabled))))
 
     def set_chunking(self, max_chunks: int):
-        """Cap the panel chunks per tile (1: every task walks the whole panel)."""
+        """Cap the panel chunks per tile (1: every task walks the whole panel;
+        1024, the most: the default)."""
         _check(self._lib, self._lib.esg_scorer_set_chunking(self._h, int(max_chunks)))
 
     def scores_len(self, n: int) -> bool:

@@ -222,9 +222,10 @@ esg_status esg_scorer_set_split(esg_scorer* scorer, uint32_t split_len);
  * few 32-lane tiles to keep every resident warp busy to the end (few reads,
  * or a large panel), each tile's reference pairs are cut into up to
  * `max_chunks` chunks of about equal columns, one task each, and the
- * per-chunk states are merged on the device.  1 turns it off; without this
- * call a tile has as many as the batch calls for, a reference pair each at
- * most.  Scores do not depend on it. */
+ * per-chunk states are merged on the device.  1 turns it off, 1024 is the
+ * most and the default: a tile then has as many as the batch calls for, a
+ * reference pair each at most, within 1 GiB for the states.  Scores do not
+ * depend on it. */
 esg_status esg_scorer_set_chunking(esg_scorer* scorer, uint32_t max_chunks);
 
 /* GpuScorer::scores_len (cuda/mod.rs:506-508): 1 for every len > 0 -- nothing

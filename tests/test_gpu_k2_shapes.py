@@ -7,7 +7,7 @@ first they do not."""
 import numpy as np
 import pytest
 
-from eschalign_b200 import GpuScorer, Mode, Scoring
+from eschalign_b200 import GpuError, GpuScorer, Mode, Scoring
 from tests.test_gpu_parity import check
 
 pytestmark = pytest.mark.gpu
@@ -152,3 +152,37 @@ def test_chunk_states_of_few_tiled_queries(oracle, kernel):
     assert list(got.ties[n // 2, :cap]) == list(ties[0][:cap])
     if kernel == "empty":
         assert (np.delete(got.results["flags"], n // 2) & 1).all()
+
+
+@pytest.mark.parametrize("merge", ["fused", "unfused"])
+def test_chunks_past_64(oracle, merge):
+    """A panel of more than 1024 reference pairs, ties spread over it, cut
+    into up to 1024 chunks: what a scorer does by itself and what
+    set_chunking(1024) gives back after a smaller cap; merged straight into
+    the results or, with a read on the int32 lanes in the batch, apart."""
+    rng = np.random.default_rng(1024)
+    same = rng.integers(0, 4, 12).astype(np.uint8)
+    panel = [same if k % 7 == 0 else rng.integers(0, 4, int(rng.integers(8, 14))).astype(np.uint8)
+             for k in range(2101)]
+    panel[7] = rng.integers(0, 4, 40).astype(np.uint8)
+    sc, cap = (2, -1, -10, -1000), 32
+    reads = [same.copy(), rng.integers(0, 4, 9).astype(np.uint8), np.zeros(0, np.uint8)]
+    if merge == "unfused":
+        reads.append(rng.integers(0, 4, 30).astype(np.uint8))  # past the semi-global lanes
+    want, ties, _ = oracle.scalar_map_batch(reads, panel, sc, False, True, cap=cap)
+    with GpuScorer(panel, Scoring(*sc), Mode.SEMIGLOBAL, tie_capacity=cap) as g:
+        for bad in (0, 1025):
+            with pytest.raises(GpuError):
+                g.set_chunking(bad)
+        for chunks in (None, 1, 64, 1024):
+            if chunks:
+                g.set_chunking(chunks)
+            got = g.score_batch(reads, both_strands=True)
+            assert got.stats["panel_chunks"] == (chunks or 1024)
+            assert got.stats["queries_plain"] == (2 if merge == "unfused" else 0)
+            for f in ("best", "suboptimal", "n_tied"):
+                assert (got.results[f] == want[f]).all(), (chunks, f)
+            for k in range(len(reads)):
+                m = min(int(want["n_tied"][k]), cap)
+                assert list(got.ties[k, :m]) == list(ties[k][:m]), (chunks, k)
+                assert (got.ties[k, m:] == 0xFFFFFFFF).all()
