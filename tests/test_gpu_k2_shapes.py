@@ -186,3 +186,24 @@ def test_chunks_past_64(oracle, merge):
                 m = min(int(want["n_tied"][k]), cap)
                 assert list(got.ties[k, :m]) == list(ties[k][:m]), (chunks, k)
                 assert (got.ties[k, m:] == 0xFFFFFFFF).all()
+
+
+@pytest.mark.parametrize("scoring", [(100, -27, -7, -1), (120, -7, -7, -1), (64, -63, 0, 0),
+                                     (127, 0, 0, -1), (23, -104, 0, -1), (89, -38, -30, -2)])
+def test_f16_lanes_up_to_their_table_and_score(oracle, scoring):
+    """Schemes whose largest table byte is the last that fits (match less a
+    negative mismatch 127; 23, -104 reaches it with the largest offset), panels
+    whose largest score is the last one the f16 lanes hold and one base more,
+    all taken by the batched kernel."""
+    match = scoring[0]
+    assert match - min(scoring[1], 0) == 127
+    rng = np.random.default_rng(match)
+    for length in (2047 // match, 2047 // match + 1):
+        panel = [rng.integers(0, 4, length).astype(np.uint8) for _ in range(3)]
+        panel.append(np.full(length, 4, np.uint8))  # wildcards: every read scores the most
+        reads = _reads(rng, panel, [length, length - 1, length + 40, 5, 300, 1100])
+        reads += [p.copy() for p in panel]
+        with GpuScorer(panel, Scoring(*scoring), Mode.LOCAL) as g:
+            assert g.info()["batched_ok"]
+            assert g.prepare(reads, both_strands=True).work_split() == (2 * len(reads), 0)
+        check(oracle, panel, reads, scoring, Mode.LOCAL, "f16 limit", kernels=DEFAULT)
