@@ -350,6 +350,7 @@ __global__ void __launch_bounds__(kTThreads) k7_trace(const K7Params P) {
 constexpr int kTagRows = 1024;    // longest read
 constexpr int kTagCols = 1700;    // longest reference: 592 warps' scratch in kTagBytes
 constexpr uint64_t kTagBytes = 2ull << 30;
+constexpr uint64_t kTagOwn = 64ull << 20;  // scratch up to this: the scorer's own pool
 constexpr int kTagScore = 30000;  // bound on |score|, gap floors included
 constexpr int kAhead = 8;         // cells of the walk read at once (4, 8, 16: 1.24, 1.19, 1.27 ms)
 constexpr int kTagNeg = -31000 * 65536;
@@ -905,13 +906,13 @@ esg_status align_impl(esg_scorer* sc, const uint8_t* d_codes, const uint64_t* d_
   const size_t tag_bytes = (size_t)tag_steps * 128 * sizeof(uint4);
   const uint64_t blocks = grid(fn, n_full, trace_words * 8, 4ull << 30);
   // k7_tags' scratch: the least of 512 MiB, 1 and 2 GiB that holds four warps
-  // an SM, and all of it once a call needs half (what the shared pool keeps
-  // then fits the next call, whose jobs need a little more)
+  // an SM, in eighths of it (what the shared pool keeps then fits the next
+  // call, whose jobs need a little more)
   uint64_t tag_room = kTagBytes / 4;
   while (tag_room < kTagBytes && tag_room / tag_bytes < 4ull * P.sm_count) tag_room *= 2;
   const uint64_t tag_blocks = grid(tag_fn, n_tag, tag_bytes, tag_room);
   const uint64_t tag_need = tag_blocks * kTWarps * tag_bytes;
-  const uint64_t tag_alloc = tag_need > tag_room / 2 ? std::max(tag_need, tag_room) : tag_need;
+  const uint64_t tag_alloc = (tag_need + tag_room / 8 - 1) / (tag_room / 8) * (tag_room / 8);
   const uint64_t warps = blocks * kTWarps;
   const size_t scratch = warps * trace_words * 8;
 
@@ -994,10 +995,14 @@ esg_status align_impl(esg_scorer* sc, const uint8_t* d_codes, const uint64_t* d_
     K.ops = d_staging;
     if (n_tag) {
       // its scratch comes from a pool the device's scorers share: mapping it
-      // anew for each of them took longer (25 ms for 0.6 GB) than the tracing
+      // anew for each of them took longer (25 ms for 0.6 GB) than the tracing.
+      // Small scratch from the scorer's own: making the shared pool takes 0.3 ms
+      // of a first call (1000 jobs: 0.8 ms, 1.2 with it)
+      const bool own = tag_need <= kTagOwn;
       uint4* d_tags = nullptr;
-      TCUDA(cudaMallocFromPoolAsync((void**)&d_tags, tag_alloc,
-                                    esg_internal_trace_pool(P.device, kTagBytes, P.pool), st));
+      TCUDA(cudaMallocFromPoolAsync(
+          (void**)&d_tags, own ? tag_need : tag_alloc,
+          own ? P.pool : esg_internal_trace_pool(P.device, kTagBytes, P.pool), st));
       K7TagParams T{K, d_tags, tag_steps, 1};
       T.J.n_tasks = n_tag;
       T.J.task_counter = d_counter;
