@@ -999,16 +999,22 @@ esg_status align_impl(esg_scorer* sc, const uint8_t* d_codes, const uint64_t* d_
       // Small scratch from the scorer's own: making the shared pool takes 0.3 ms
       // of a first call (1000 jobs: 0.8 ms, 1.2 with it)
       const bool own = tag_need <= kTagOwn;
+      cudaMemPool_t pool = own ? P.pool : esg_internal_trace_pool(P.device, kTagBytes, P.pool);
+      uint64_t ctas = tag_blocks, bytes = own ? tag_need : tag_alloc;
       uint4* d_tags = nullptr;
-      TCUDA(cudaMallocFromPoolAsync(
-          (void**)&d_tags, own ? tag_need : tag_alloc,
-          own ? P.pool : esg_internal_trace_pool(P.device, kTagBytes, P.pool), st));
+      cudaError_t e = cudaMallocFromPoolAsync((void**)&d_tags, bytes, pool, st);
+      while (e == cudaErrorMemoryAllocation && ctas > 1) {
+        cudaGetLastError();  // short of memory: fewer warps take the tasks
+        ctas = (ctas + 1) / 2;
+        bytes = ctas * kTWarps * tag_bytes;
+        e = cudaMallocFromPoolAsync((void**)&d_tags, bytes, pool, st);
+      }
+      TCUDA(e);
       K7TagParams T{K, d_tags, tag_steps, 1};
       T.J.n_tasks = n_tag;
       T.J.task_counter = d_counter;
       void* args[] = {&T};
-      const cudaError_t e =
-          cudaLaunchKernel(tag_fn, dim3((unsigned)tag_blocks), dim3(kTThreads), args, 0, st);
+      e = cudaLaunchKernel(tag_fn, dim3((unsigned)ctas), dim3(kTThreads), args, 0, st);
       cudaFreeAsync(d_tags, st);
       TCUDA(e);
     }

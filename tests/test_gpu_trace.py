@@ -231,3 +231,23 @@ def test_trace_leading_deletion_by_hand(oracle):
         rec = got.records[0]
         assert (int(rec["score"]), got.cigar(0), int(rec["query_start"]), int(rec["query_end"]),
                 int(rec["ref_start"]), int(rec["ref_end"])) == (score, "3D20M", 5, 25, 0, 23)
+
+
+def test_trace_short_of_device_memory():
+    """With 300 MiB of device memory left, jobs whose scratch would be 512 MiB
+    run on fewer warps, to the same records."""
+    import torch
+    refs = synth.panel_tiles()
+    reads = synth.reads_c2(refs, n=20_000, seed=0x5EED_0B0E).tuple()
+    jobs = [(k, k % len(refs), k & 1) for k in range(20_000)]
+    with GpuScorer(refs, Scoring(), Mode.SEMIGLOBAL) as g:
+        want = g.align(reads, jobs)
+    with GpuScorer(refs, Scoring(), Mode.SEMIGLOBAL) as g:
+        hog = torch.empty(torch.cuda.mem_get_info()[0] - (300 << 20), dtype=torch.uint8,
+                          device="cuda")
+        try:
+            got = g.align(reads, jobs)
+        finally:
+            del hog
+            torch.cuda.empty_cache()
+    assert np.array_equal(got.records, want.records) and np.array_equal(got.ops, want.ops)
