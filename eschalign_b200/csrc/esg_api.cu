@@ -1515,6 +1515,21 @@ cudaMemPool_t esg_internal_trace_pool(int device, uint64_t keep, cudaMemPool_t o
   return t.pool;
 }
 
+size_t esg_internal_trace_trim(int device) {
+  if (device < 0 || device >= kMaxDevices) return 0;
+  std::lock_guard<std::mutex> lk(g_trace_mu);
+  const cudaMemPool_t pool = g_trace[device].pool;
+  uint64_t before = 0, after = 0;
+  if (!pool ||
+      cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, &before) != cudaSuccess ||
+      cudaMemPoolTrimTo(pool, 0) != cudaSuccess ||
+      cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, &after) != cudaSuccess) {
+    cudaGetLastError();
+    return 0;
+  }
+  return before > after ? (size_t)(before - after) : 0;
+}
+
 int esg_internal_device(const esg_scorer* sc) { return sc ? sc->device : 0; }
 
 uint32_t esg_internal_tie_capacity(const esg_scorer* sc) { return sc ? sc->cap : 0; }

@@ -37,6 +37,8 @@ ESG_HIDDEN void esg_internal_panel_of(esg_scorer* sc, esg_internal_panel* out);
 // scorers, keeping up to `keep` bytes between calls, gone with the last of
 // them.  `other` if it cannot be made.
 ESG_HIDDEN cudaMemPool_t esg_internal_trace_pool(int device, uint64_t keep, cudaMemPool_t other);
+// Give back what that pool keeps and no traceback uses; returns the bytes.
+ESG_HIDDEN size_t esg_internal_trace_trim(int device);
 
 // A submitted batch's reads on the device (NULL codes if not submitted).
 ESG_HIDDEN void esg_internal_batch_reads(const esg_batch* b, const uint8_t** codes,

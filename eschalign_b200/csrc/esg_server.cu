@@ -11,9 +11,10 @@
 // Admission: under the server lock, a batch of B device bytes is admitted
 // when B fits the free device memory (cudaMemGetInfo) plus the spare memory
 // of the scorer's pool, less the headroom, and, with a budget, the bytes of
-// admitted batches plus B stay within it.  Otherwise the worker first
-// finishes its own oldest batch, or with none in flight waits for other
-// slots to release memory.  A batch that could not fit even on an idle
+// admitted batches plus B stay within it.  Otherwise the worker has the
+// device's traceback pool give back what it keeps, then finishes its own
+// oldest batch, or with none in flight waits for other slots to release
+// memory.  A batch that could not fit even on an idle
 // device (B above the budget, or above total memory less the headroom) is
 // refused: its requests end with ESG_ERR_OUT_OF_MEMORY.  All of this is
 // host logic; nothing waits on the device except esg_finish.
@@ -286,7 +287,7 @@ void worker(esg_server* sv, Slot* sp) {
     esg_batch_stats_get(b, &bst);
     const uint64_t need = bst.device_bytes;
     // admission
-    bool refused = false;
+    bool refused = false, trimmed = false;
     // with nothing of the server's in flight, memory held outside the server
     // may never come back: give up after this long
     const auto give_up = Clock::now() + std::chrono::seconds(5);
@@ -309,6 +310,12 @@ void worker(esg_server* sv, Slot* sp) {
         sv->stats.peak_bytes_in_flight =
             std::max(sv->stats.peak_bytes_in_flight, sv->stats.bytes_in_flight);
         break;
+      }
+      if (!mem_ok && !trimmed) {  // what tracebacks keep between calls
+        trimmed = true;
+        lk.unlock();
+        if (esg_internal_trace_trim(esg_internal_device(s.scorer))) continue;
+        lk.lock();
       }
       sv->stats.admission_waits++;
       if (!s.inflight.empty()) {  // release our own memory first

@@ -400,7 +400,10 @@ typedef struct esg_alignment {
 /* Trace `jobs` against the reads of a submitted batch (its reads are still
  * on the device: call after esg_finish, before esg_batch_free).  `ops`
  * holds ops_capacity words; ESG_ERR_BAD_ARGUMENT if the alignments need
- * more (the needed count is then in *ops_needed, which may be NULL). */
+ * more (the needed count is then in *ops_needed, which may be NULL).  Device
+ * scratch past 64 MiB comes from a pool that the device's scorers share; it
+ * keeps up to 2 GiB between calls, gives it back when a server's admission
+ * runs short (esg_server_new), and goes with the last scorer. */
 esg_status esg_align_batch(esg_scorer* scorer, esg_batch* batch, const esg_align_job* jobs,
                            uint32_t n_jobs, esg_alignment* out, uint32_t* ops,
                            uint64_t ops_capacity, uint64_t* ops_needed);

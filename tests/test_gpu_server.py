@@ -154,3 +154,26 @@ def test_server_splits_large_requests_into_pieces():
     assert tms.total_ms <= tmb.total_ms  # the small one did not wait for all of the big one
     g.close()
     solo.close()
+
+
+def test_server_admission_takes_back_what_tracebacks_keep():
+    """A traceback's scratch (512 MiB here) stays in a pool of the device's
+    scorers: a batch that fits the memory only without it is admitted."""
+    import torch
+    from eschalign_b200 import synth
+    refs = synth.panel_tiles()
+    reads = synth.reads_c2(refs, n=20_000, seed=0x5EED_0B0F)
+    jobs = [(k, k % len(refs), k & 1) for k in range(20_000)]
+    tracer = GpuScorer(refs, Scoring(*SCORING), Mode.SEMIGLOBAL)
+    g = GpuScorer(refs, Scoring(*SCORING), Mode.LOCAL, tie_capacity=CAP)
+    want = g.score_batch(reads.slice(0, 10).tuple())
+    tracer.align(reads.tuple(), jobs)
+    free = torch.cuda.mem_get_info()[0]
+    with Server([g], memory_headroom=free + (256 << 20)) as sv:
+        res, _ = sv.wait(sv.submit(0, reads.slice(0, 10).list(), False), 60_000)
+        assert sv.stats()["refused"] == 0
+    assert np.array_equal(res.results["best"], want.results["best"])
+    assert torch.cuda.mem_get_info()[0] >= free + (256 << 20)
+    tracer.align(reads.slice(0, 10).tuple(), jobs[:10])  # and tracing goes on
+    tracer.close()
+    g.close()
