@@ -94,9 +94,20 @@ constexpr uint32_t kMaxChunks = 1024;
 // Device memory the panel chunks' states may take (per batch).
 constexpr uint64_t kPartBudget = 1ull << 30;
 
-// A batch's device counters: [1] re-score requests, [2] error bits, [6..7]
-// k3's 64-bit unit counter, one task counter per k2 shape in the others.
-constexpr uint32_t kCounters = 9;
+// A batch's device counters: re-score requests, error bits, k3's 64-bit unit
+// counter (two words, 8-byte aligned) and a task counter per k2 shape.
+enum Counter {
+  kTasks16 = 0,
+  kRedoCount,
+  kErrorBits,
+  kTasksLong,
+  kTasks32,
+  kTasks28,
+  kUnitsInt32,
+  kTasks8 = kUnitsInt32 + 2,
+  kCounters
+};
+constexpr int kTaskCounter[kShapes] = {kTasksLong, kTasks32, kTasks28, kTasks16, kTasks8};
 
 // Pinned host memory, reused across batches of one scorer.
 struct PinnedPool {
@@ -1292,10 +1303,11 @@ static esg_status prepare_impl(esg_scorer* sc, const uint8_t* const* ptrs, const
   b->n_q = n_reads * (both ? 2u : 1u);
   b->total_bases = total;
 
-  // --- plan: which queries go where.  Short queries take 16-row stripes,
-  // longer ones 32-row stripes (from sc->split_len, set by the autotuner),
-  // queries over 32 stripes of 32 rows run alone in passes; what the
-  // batched kernel cannot take goes to the int32 kernel.
+  // --- plan: which queries go where.  Queries up to sc->split_len (set by
+  // the autotuner) take 16-row stripes, longer ones what shape_of gives (28 or
+  // 32 rows; over 32 stripes of 32 rows, alone in passes), those of a small
+  // batch 8 or 16 rows (below); what the batched kernel cannot take goes to
+  // the int32 kernel.
   std::vector<std::pair<uint32_t, uint32_t>> qs[kShapes];  // (stripes, query)
   std::vector<uint8_t> route(b->n_q, 0);  // 0 empty or k2, 2 k3
   bool sg_check = false, half[kShapes] = {true, true, true, true, true};
@@ -1444,7 +1456,7 @@ static esg_status prepare_impl(esg_scorer* sc, const uint8_t* const* ptrs, const
   }
   // the packed tail up to the last whole word unpacks to padding
   memset(b->h_packed + pos / 4, 0, b->code_words * 4 - pos / 4);
-  // order[] and tasks[] laid out [long | 32-row tiles | 16-row tiles];
+  // order[] and tasks[] laid out by shape (K2Shape's order);
   // tasks[t] = {start in order[], count | stripes << 16}
   {
     uint32_t lanes = 0, o = 0, t = 0;
@@ -1682,8 +1694,7 @@ static esg_status launch_device_work(esg_scorer* sc, esg_batch* b, cudaStream_t 
       K2Params T = P;
       T.tasks = P.tasks + tile0;
       T.n_tasks = b->n_tiles[k] * nc;
-      static const int kCounter[kShapes] = {3, 4, 5, 0, 1 + 7};
-      T.task_counter = b->d_counters + kCounter[k];
+      T.task_counter = b->d_counters + kTaskCounter[k];
       const auto& kn = sc->k2[k][second(T, b->second[k])];
       void* targs[] = {&T};
       ESG_CUDA(cudaLaunchKernel(kn.fn, dim3(grid(kn.blocks, T.n_tasks)), dim3(kK2Threads), targs,
@@ -1726,7 +1737,7 @@ static esg_status launch_device_work(esg_scorer* sc, esg_batch* b, cudaStream_t 
     P.n_reads = b->n_reads;
     P.list = b->d_list;
     P.host_count = b->host_list;
-    P.redo_count = b->redo_cap ? b->d_counters + 1 : nullptr;
+    P.redo_count = b->redo_cap ? b->d_counters + kRedoCount : nullptr;
     P.redo_cap = b->redo_cap;
     P.rcodes = sc->d_rcodes;
     P.roff = sc->d_roff;
@@ -1740,9 +1751,9 @@ static esg_status launch_device_work(esg_scorer* sc, esg_batch* b, cudaStream_t 
     const int k3_blocks = plain ? sc->k3_blocks1 : sc->k3_blocks;
     P.refs_per_task = k3_refs_per_task((uint64_t)b->host_list + b->redo_cap, sc->n_refs,
                                        (uint64_t)k3_blocks * kK3Warps);
-    // counters[6..7]: the units' 64-bit counter (8-byte aligned, reset with
-    // the rest each launch)
-    P.task_counter = reinterpret_cast<unsigned long long*>(b->d_counters + 6);
+    // (8-byte aligned, reset with the rest each launch)
+    static_assert(kUnitsInt32 % 2 == 0, "the 64-bit counter's alignment");
+    P.task_counter = reinterpret_cast<unsigned long long*>(b->d_counters + kUnitsInt32);
     P.colbuf = plain ? sc->d_colbuf1 : sc->d_colbuf;
     P.ma = sc->scoring.match_score;
     P.mi = sc->scoring.mismatch;
@@ -1833,8 +1844,8 @@ static uint32_t work_key(const esg_scorer* sc, const esg_batch* b) {
 }
 
 // The batch's device work as one CUDA graph launch on `st`: the launch
-// sequence (counter reset, the three k2 groups on two streams joined by
-// events, chunk merge, k3 / k4, k5, k6) is captured from the scorer's
+// sequence (counter reset, k2's shapes on two streams joined by events, chunk
+// merge, k3 / k4, k5, k6) is captured from the scorer's
 // stream once per batch, and the scorer's instantiated graph of that shape
 // is updated with the batch's parameters and launched.  Work already in
 // flight from an earlier launch of the same graph keeps its own parameters.
@@ -2023,8 +2034,8 @@ esg_status esg_finish(esg_scorer* sc, esg_batch* b, esg_read_result* results, ui
   ESG_CUDA(cudaSetDevice(sc->device));
   ESG_CUDA(cudaEventSynchronize(b->done));
   ESG_CUDA(cudaGetLastError());
-  const uint32_t errbits = b->h_counters[2];
-  b->stats.queries_rescored = std::min(b->h_counters[1], b->redo_cap);
+  const uint32_t errbits = b->h_counters[kErrorBits];
+  b->stats.queries_rescored = std::min(b->h_counters[kRedoCount], b->redo_cap);
   if (errbits & kErrPanelWait)
     return fail(ESG_ERR_TIMEOUT, "the panel's shared-memory staging did not complete");
   if (errbits & kErrRedoOverflow)

@@ -36,7 +36,6 @@
 
 namespace esg {
 
-constexpr int kRows = 16;             // rows per lane stripe (k2)
 constexpr int kMaxStripes = 32;       // a query spans at most one warp (k2)
 constexpr int kNeg16 = -31500;        // int16 stand-in for -infinity (biased domain)
 constexpr int kBiasLocal = 2048;      // local: H + B >= B >= |o|, |e|
@@ -113,11 +112,6 @@ __device__ __forceinline__ uint32_t ld_shared_u32(uint32_t addr) {
   uint32_t v;
   asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(addr));
   return v;
-}
-__device__ __forceinline__ uint32_t add16x2(uint32_t a, uint32_t b) {
-  uint32_t d;
-  asm("add.s16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
-  return d;
 }
 // a * b + c as a 32-bit IMAD, which issues to the FMA pipe and so keeps the
 // integer ALU free for the DPX ops
