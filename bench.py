@@ -19,12 +19,15 @@ other three (mode, scheme) combinations are measured once each.
             batches in flight, like eschalign's GPU feeder thread
             (crates/eschalign-cli/src/align.rs:2801-2917), host<->device
             copies inside the timed region.
-* roofline  integer ALU: the batched kernel's algorithmic work (12 int ops a
-            cell local, 11 semi-global, two cells per 32-bit lane op) against
-            the integer lane-op peak measured by csrc/esg_probe.cu in the same
-            run.
+* roofline  integer ALU: the DPX instructions a cell pair cannot do without
+            (E, F and H, and half of one for the local best: 3.5 local up to
+            scores of 2047, 3 semi-global; the adds are on the FMA pipe)
+            against the rate at which DPX instructions issue, measured by
+            csrc/esg_probe.cu in the same run.
 * --impl reference  the reference's CPU path (AVX-512BW score kernels +
-            selection, restated in oracle/) on all host cores.
+            selection) on all host cores, as this repository restates it in C
+            (oracle/, "kind": "port"): the reference itself is Rust, for which
+            there is no toolchain here.
 
 Other workloads (``--workload``), one JSON line each, same keys:
 
@@ -71,7 +74,7 @@ import numpy as np  # noqa: E402
 HEADLINE = ((2, -1, -10, -1), "local")
 COMBOS = [((2, -1, -10, -1), "local"), ((2, -1, -10, -1), "semiglobal"),
           ((1, -1, -2, -1), "local"), ((1, -1, -2, -1), "semiglobal")]
-OPS_PER_CELL = {"local": 12, "semiglobal": 11}
+DPX_PER_CELL_PAIR = {"local": 3.5, "semiglobal": 3.0}
 C4_SCORING = (2, -1, -10, -1)
 C3_SCORING = (2, -1, -10, -1)
 # DRAM bytes per DP cell of the batched kernel: 36.95 MB read, 5.11 MB
@@ -206,20 +209,20 @@ def int_peak(device):
     ops = {lib.esg_probe_op_name(k).decode(): {"lane_ops_per_s": rates[k],
                                                 "per_sm_per_clk": per_clk[k]}
            for k in range(n.value)}
-    peak = max(ops["iadd32"]["lane_ops_per_s"], ops["imax32"]["lane_ops_per_s"])
-    return {"peak_lane_ops_per_s": peak, "ops": ops, "sms": sms.value}
+    return {"ops": ops, "sms": sms.value}
 
 
 def roofline_of(peak, per_gpu_cells_s, mode, traffic):
-    achieved = per_gpu_cells_s * OPS_PER_CELL[mode] / 2.0
+    achieved = per_gpu_cells_s * DPX_PER_CELL_PAIR[mode] / 2.0
+    rate = peak["ops"]["viaddmax16x2"]["lane_ops_per_s"] if peak else None
     return {"bound": "int_alu", "achieved": achieved / 1e12,
-            "peak": (peak["peak_lane_ops_per_s"] / 1e12) if peak else None,
-            "unit": "T lane-ops/s",
-            "frac": (achieved / peak["peak_lane_ops_per_s"]) if peak else None,
+            "peak": rate / 1e12 if rate else None,
+            "unit": "T DPX lane-instructions/s",
+            "frac": achieved / rate if rate else None,
             "traffic": traffic, "kernel": "k2_batched",
-            "note": f"achieved = cells/s x {OPS_PER_CELL[mode]} int ops / 2 cells per "
-                    "int16x2 lane-op; peak = measured iadd32/imax32 lane-op rate "
-                    "(csrc/esg_probe.cu), measured in this run"}
+            "note": f"achieved = cells/s x {DPX_PER_CELL_PAIR[mode]} DPX instructions / 2 cells "
+                    "per lane; peak = measured viaddmax.s16x2 issue rate (csrc/esg_probe.cu), "
+                    "measured in this run"}
 
 
 def cpu_baseline(refs, reads, scoring, mode, seconds, threads=0, chunk=64):
@@ -765,7 +768,8 @@ def reference_gpu_arms(refs, reads, scoring, local, device):
 
 
 def run_reference(a, rank, world):
-    """--impl reference: rank 0 times the CPU path; other ranks exit."""
+    """--impl reference: rank 0 times the CPU path, this repository's C port of
+    it; other ranks exit."""
     if rank != 0:
         return
     from eschalign_b200 import synth
@@ -838,7 +842,10 @@ def run_reference(a, rank, world):
         cells_per_read = 2 * (data.bases() / len(data)) * sum(len(r) for r in refs)
         extra["reads_per_s"] = v * 1e9 / cells_per_read
     line = {
-        "impl": "reference", "metric": "GCUPS", "value": v, "unit": "GCUPS", "n_gpus": a.gpus,
+        "impl": "reference", "kind": "port",
+        "note": "this repository's C restatement of the reference's CPU path (oracle/); the "
+                "reference is Rust, which cannot be built here",
+        "metric": "GCUPS", "value": v, "unit": "GCUPS", "n_gpus": a.gpus,
         "steps": a.steps, "warmup": a.warmup, "ms_per_step": 1e3 * last["seconds"],
         "higher_is_better": True, "scaling": "weak", "vs_baseline": None, "dtype": dtype,
         "data": "synthetic", **extra,
@@ -1451,7 +1458,8 @@ def run_c5(a, ctx, rank):
             {"value": best["gcups"], "unit": "GCUPS", "h2d_bytes_per_step": best["h2d_bytes"],
              "d2h_bytes_per_step": best["d2h_bytes"],
              "note": "serving is end to end: host requests in, results out"},
-            roofline_of(peak, best["gcups"] * 1e9, "local", None), clocks,
+            # (half the requests are local: the smaller of the two counts)
+            roofline_of(peak, best["gcups"] * 1e9, "semiglobal", None), clocks,
             int(st["kernels"]))
         line["value_note"] = ("aggregate GCUPS at the busiest rate (all requests, wall clock); "
                               "gpu_launches = kernels of every batch of the sweep")
