@@ -17,7 +17,9 @@
 #include <cstdlib>
 #include <cstring>
 #include <mutex>
+#include <new>
 #include <string>
+#include <system_error>
 #include <thread>
 #include <vector>
 
@@ -2156,12 +2158,16 @@ namespace {
 // handles).
 struct BitPlanes {
   std::vector<uint64_t> lo, hi, wild;
-  // false: a code above 4
+  // false: a code above 4, or no memory
   bool set(const uint8_t* c, uint32_t n) {
     const uint32_t words = n / 64 + 2;  // one spare: a window may straddle the last
-    lo.assign(words, 0);
-    hi.assign(words, 0);
-    wild.assign(words, 0);
+    try {
+      lo.assign(words, 0);
+      hi.assign(words, 0);
+      wild.assign(words, 0);
+    } catch (const std::bad_alloc&) {
+      return false;
+    }
     uint64_t bad = 0;
     uint32_t i = 0;
     // bit b of eight bytes to eight bits: the product's top byte collects them
@@ -2298,10 +2304,19 @@ void trim_batch(const uint8_t* codes, const uint64_t* off, const uint32_t* len, 
     work(0, n_pairs);
     return;
   }
+  // the caller takes the last share, and all that no thread can be had for
   std::vector<std::thread> th;
+  th.reserve(nt);
   const uint32_t per = (n_pairs + nt - 1) / nt;
-  for (uint32_t t = 0; t < nt; ++t)
-    th.emplace_back(work, std::min(n_pairs, t * per), std::min(n_pairs, (t + 1) * per));
+  uint32_t t = 0;
+  for (; t + 1 < nt; ++t) {
+    try {
+      th.emplace_back(work, std::min(n_pairs, t * per), std::min(n_pairs, (t + 1) * per));
+    } catch (const std::system_error&) {
+      break;
+    }
+  }
+  work(std::min(n_pairs, t * per), n_pairs);
   for (auto& x : th) x.join();
 }
 

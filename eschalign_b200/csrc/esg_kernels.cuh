@@ -1,6 +1,6 @@
 // esg_kernels.cuh -- device code of the B200 panel scorer (sm_100a).
 //
-// Four kernels, launched in this order on one stream per batch:
+// The kernels, in the order a batch launches them:
 //
 //   k2_batched   the product: every (query, reference pair) of the panel in
 //                16-bit lanes.  One warp is a 32-lane systolic array: each
@@ -19,7 +19,7 @@
 //                is re-scored by the int32 kernel.
 //   k3_lanes     the exact int32 path: the recurrence of
 //                crates/eschalign/src/scalar.rs:120-163 on chains of lanes
-//                (16-row stripes, bottom rows passed by shuffle, several
+//                (28- or 32-row stripes, bottom rows passed by shuffle, several
 //                references a warp for short queries); what k2 cannot take
 //                or flags.  With one lane a chain it is the one-thread-per-
 //                pair comparison arm.
