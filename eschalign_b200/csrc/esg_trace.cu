@@ -169,6 +169,8 @@ __global__ void __launch_bounds__(kTThreads) k7_trace(const K7Params P) {
         E[r] = kNegT;
       }
       int hbot = 0, fbot = kNegT, hdg = 0;
+      // the pass's first maximum (its columns come in order)
+      int pb = kLocal ? 0 : kNegT, pj = 0, pi = 0;
       const int skew = long_job ? lane : s;
       int steps = valid ? m + skew : 0;
 #pragma unroll
@@ -215,10 +217,10 @@ __global__ void __launch_bounds__(kTThreads) k7_trace(const K7Params P) {
             hdiag = hleft;
             H[r] = h;
             hup = h;
-            if (kLocal && h > best) {  // pad rows hold 0: never above best
-              best = h;
-              bi = s * kTR + r - pad + 1;
-              bj = j + 1;
+            if (kLocal && h > pb) {  // pad rows hold 0: never above it
+              pb = h;
+              pi = s * kTR + r - pad + 1;
+              pj = j + 1;
             }
           }
           trace[((size_t)pass * P.mcols + j) * 32 + lane] = make_uint2(w0, w1);
@@ -227,24 +229,30 @@ __global__ void __launch_bounds__(kTThreads) k7_trace(const K7Params P) {
           if (to_buf) colbuf[j] = make_uint2((uint32_t)hbot, (uint32_t)fbot);
           if (!kLocal) {
             if (j < m - 1) {
-              if (s == S - 1 && hbot > best) {  // the last row
-                best = hbot;
-                bi = (int)n;
-                bj = j + 1;
+              if (s == S - 1 && hbot > pb) {  // the last row
+                pb = hbot;
+                pi = (int)n;
+                pj = j + 1;
               }
             } else {
 #pragma unroll
               for (int r = 0; r < kTR; ++r) {  // the last column, rows in order
                 const int i = s * kTR + r - pad + 1;
-                if (i >= 1 && H[r] > best) {
-                  best = H[r];
-                  bi = i;
-                  bj = m;
+                if (i >= 1 && H[r] > pb) {
+                  pb = H[r];
+                  pi = i;
+                  pj = m;
                 }
               }
             }
           }
         }
+      }
+      // (a later pass starts at the first column again)
+      if (better(pb, pj, pi, best, bj, bi)) {
+        best = pb;
+        bj = pj;
+        bi = pi;
       }
       __syncwarp();  // trace and column buffer writes visible to the warp
     }

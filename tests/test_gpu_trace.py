@@ -251,3 +251,35 @@ def test_trace_short_of_device_memory():
             del hog
             torch.cuda.empty_cache()
     assert np.array_equal(got.records, want.records) and np.array_equal(got.ops, want.ops)
+
+
+@pytest.mark.parametrize("mode", [Mode.LOCAL, Mode.SEMIGLOBAL])
+@pytest.mark.parametrize("n,scoring", [(600, (1000, 0, -300, -300)), (1100, (2, 0, -3, -1)),
+                                       (1700, (2, 0, -3, -1)), (2600, (5, 0, -9, -2))])
+def test_trace_equal_ends_in_two_passes(oracle, mode, n, scoring):
+    """A long read's passes each walk every column: of equal ends in two
+    passes, rows a whole number of passes (512 rows) apart, the one in the
+    smaller column is the alignment's, whichever pass it is in."""
+    a, b = encode("ACCACAACCA"), encode("CAAACCACCC")
+    t, g = encode("T" * 20), encode("G" * n)
+    reads, panel = [], []
+    if mode == Mode.LOCAL:
+        panel = [np.concatenate([a, t, b]), np.concatenate([b, t, a])]
+        for at in (3, 60, 70):
+            for apart in range(512, n - at - 10, 512):
+                r = g.copy()
+                r[at:at + 10], r[at + apart:at + apart + 10] = b, a
+                reads.append(r)
+    else:
+        # the last row ends in column 1, a row of an earlier pass in the last
+        panel = [np.concatenate([encode("A"), t, encode("C")])]
+        for apart in range(512, n, 512):
+            r = g.copy()
+            r[n - 1 - apart], r[n - 1] = 1, 0
+            reads.append(r)
+    jobs = [(i, r, 0) for i in range(len(reads)) for r in range(len(panel))]
+    with GpuScorer(panel, Scoring(*scoring), mode) as sc:
+        got = check(oracle, sc, reads, panel, jobs, scoring, mode == Mode.LOCAL,
+                    f"passes {mode.label} {n}")
+    if mode == Mode.SEMIGLOBAL:
+        assert all(int(r["ref_end"]) == 1 and int(r["query_end"]) == n for r in got.records)
